@@ -18,6 +18,7 @@
 #include "edit_common.cuh"
 #include "voxel_b200_device.cuh"
 #include "graph.cuh"
+#include "plain.cuh"
 #include "profile.cuh"
 #include "tuning.cuh"
 
@@ -28,6 +29,7 @@
 #include <cstdio>
 #include <cmath>
 #include <new>
+#include <type_traits>
 #include <vector>
 
 namespace vx::dag {
@@ -609,100 +611,145 @@ __global__ void read_leaves_kernel(vx_dag_view v, uint32_t lx0, uint32_t ly0, ui
 
 // ------------------------------------------------------- plain path prep --
 
-// Voxel -> (leaf key, bit).  The key is the leaf's Morton path, 3 bits per
-// inner level with the root's child in the top bits (the reference's
-// make_leaf_key, hash_dag_gpu/detail/node.cuh:67-85, widened to 64 bits);
-// voxels outside the world get key 1 << (3 * depth) and are dropped.
-__global__ void pack_voxels_kernel(const vx_voxel *v, uint32_t n, uint32_t depth,
-                                   uint64_t *keys, uint32_t *bits) {
+// Leaf keys: the leaf's Morton path, 3 bits per inner level with the root's
+// child in the top bits (the reference's make_leaf_key, hash_dag_gpu/detail/
+// node.cuh:67-85, widened to 64 bits).  Lists keep them in 32-bit words when
+// they fit (depth <= 10, with the bit that marks leaves outside the world),
+// which halves the key traffic of the sort: 8.78 M voxels at depth 10 sort in
+// 0.32 ms with 32-bit keys against 0.40 ms with 64-bit ones on B200.
+constexpr uint32_t kMaxDepthKey32 = 10;
+
+// Bits of v moved to every third bit (v < 2^10 for u32, < 2^21 for u64) and
+// back.
+__device__ __forceinline__ uint32_t spread3(uint32_t v) {
+  v = (v | (v << 16)) & 0x030000ffu;
+  v = (v | (v << 8)) & 0x0300f00fu;
+  v = (v | (v << 4)) & 0x030c30c3u;
+  return (v | (v << 2)) & 0x09249249u;
+}
+__device__ __forceinline__ uint64_t spread3(uint64_t v) {
+  v = (v | (v << 32)) & 0x001f00000000ffffull;
+  v = (v | (v << 16)) & 0x001f0000ff0000ffull;
+  v = (v | (v << 8)) & 0x100f00f00f00f00full;
+  v = (v | (v << 4)) & 0x10c30c30c30c30c3ull;
+  return (v | (v << 2)) & 0x1249249249249249ull;
+}
+__device__ __forceinline__ uint32_t compact3(uint64_t v) {
+  v &= 0x1249249249249249ull;
+  v = (v | (v >> 2)) & 0x10c30c30c30c30c3ull;
+  v = (v | (v >> 4)) & 0x100f00f00f00f00full;
+  v = (v | (v >> 8)) & 0x001f0000ff0000ffull;
+  v = (v | (v >> 16)) & 0x001f00000000ffffull;
+  return static_cast<uint32_t>(v | (v >> 32)) & 0x1fffffu;
+}
+template <class K>
+__device__ __forceinline__ K leaf_key(uint32_t lx, uint32_t ly, uint32_t lz) {
+  return spread3(K(lx)) | (spread3(K(ly)) << 1) | (spread3(K(lz)) << 2);
+}
+
+// Voxel -> (leaf key, bit); voxels outside the world get key 1 << (3 * depth)
+// and are dropped.
+template <class K>
+__global__ void pack_voxels_kernel(const vx_voxel *v, uint32_t n, uint32_t depth, K *keys,
+                                   uint32_t *bits) {
   const uint64_t i = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x;
   if (i >= n) return;
   const vx_voxel p = v[i];
   const uint32_t side_exp = depth + 2;
-  if ((p.x >> side_exp) | (p.y >> side_exp) | (p.z >> side_exp)) {
-    keys[i] = 1ull << (3 * depth);
-    bits[i] = 0;
-    return;
-  }
-  uint64_t key = 0;
-  for (uint32_t l = 0; l < depth; ++l) {
-    const uint32_t s = side_exp - 1 - l;
-    key = (key << 3) | (((p.x >> s) & 1u) | (((p.y >> s) & 1u) << 1) | (((p.z >> s) & 1u) << 2));
-  }
-  keys[i] = key;
-  bits[i] = (p.x & 3u) + 4u * (p.y & 3u) + 16u * (p.z & 3u);
+  const bool outside = ((p.x >> side_exp) | (p.y >> side_exp) | (p.z >> side_exp)) != 0;
+  keys[i] = outside ? K(1) << (3 * depth) : leaf_key<K>(p.x >> 2, p.y >> 2, p.z >> 2);
+  bits[i] = outside ? 0u : (p.x & 3u) + 4u * (p.y & 3u) + 16u * (p.z & 3u);
 }
 
-__global__ void run_flags_kernel(const uint64_t *keys, uint32_t n, uint32_t depth,
-                                 uint32_t *flags) {
+template <class K>
+__global__ void run_flags_kernel(const K *keys, uint32_t n, uint32_t depth, uint32_t *flags) {
   const uint64_t i = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x;
   if (i >= n) return;
-  const bool valid = keys[i] < (1ull << (3 * depth));
+  const bool valid = keys[i] < (K(1) << (3 * depth));
   flags[i] = (valid && (i == 0 || keys[i - 1] != keys[i])) ? 1u : 0u;
 }
 
 // Leaf edit command -> (leaf key, command index); leaves outside the world
 // get key 1 << (3 * depth) and are dropped.
+template <class K>
 __global__ void pack_leaf_commands_kernel(const vx_leaf_command *c, uint32_t n, uint32_t depth,
-                                          uint64_t *keys, uint32_t *index) {
+                                          K *keys, uint32_t *index) {
   const uint64_t i = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x;
   if (i >= n) return;
   const vx_leaf_command cmd = c[i];
   index[i] = static_cast<uint32_t>(i);
-  if ((cmd.leaf_x >> depth) | (cmd.leaf_y >> depth) | (cmd.leaf_z >> depth)) {
-    keys[i] = 1ull << (3 * depth);
-    return;
-  }
-  uint64_t key = 0;
-  for (uint32_t l = 0; l < depth; ++l) {
-    const uint32_t s = depth - 1 - l;
-    key = (key << 3) | (((cmd.leaf_x >> s) & 1u) | (((cmd.leaf_y >> s) & 1u) << 1) |
-                        (((cmd.leaf_z >> s) & 1u) << 2));
-  }
-  keys[i] = key;
+  const bool outside =
+      ((cmd.leaf_x >> depth) | (cmd.leaf_y >> depth) | (cmd.leaf_z >> depth)) != 0;
+  keys[i] = outside ? K(1) << (3 * depth) : leaf_key<K>(cmd.leaf_x, cmd.leaf_y, cmd.leaf_z);
 }
 
-// Each run start ORs its run's voxel bits (a voxel list) or its commands'
-// masks (leaf edit commands, selected by index) into one leaf-mask primitive.
-template <bool Commands>
-__global__ void reduce_runs_kernel(const uint64_t *keys, const uint32_t *bits,
-                                   const vx_leaf_command *cmds,
-                                   const uint32_t *offsets, uint32_t n,
-                                   uint32_t depth, uint32_t op, uint32_t material,
-                                   vx_primitive *out, uint32_t *out_count) {
+// Each run of equal keys ORs its voxel bits (a voxel list) or its commands'
+// masks (leaf edit commands, selected by index) into one leaf-mask primitive,
+// written with its key by the run's first lane.  A warp takes 32 entries: the
+// ORs run over the warp by shuffles, and the run that its last entry belongs
+// to is followed past the warp's end 32 entries at a time (by the warp that
+// holds its start), so neither dense lists (runs of 64) nor heavy duplicates
+// leave one lane walking a run alone: 0.27 -> 0.08 ms for the 8.78 M
+// voxels of a sphere of radius 128 on B200.
+template <class K, bool Commands>
+__global__ void reduce_runs_kernel(const K *keys, const uint32_t *bits,
+                                   const vx_leaf_command *cmds, const uint32_t *offsets,
+                                   uint32_t n, uint32_t depth, uint32_t op, uint32_t material,
+                                   vx_primitive *out, uint64_t *leaf_keys, uint32_t *out_count) {
   const uint64_t i = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x;
+  const uint32_t lane = lane_id();
+  const uint64_t w0 = i - lane;
+  if (w0 >= n) return;
+  const K outside = K(1) << (3 * depth);
+  auto mask_of = [&](uint64_t j) {
+    if constexpr (Commands) {
+      const vx_leaf_command &c = cmds[bits[j]];
+      return static_cast<uint64_t>(c.voxel_data_low) |
+             (static_cast<uint64_t>(c.voxel_data_high) << 32);
+    } else {
+      return 1ull << bits[j];
+    }
+  };
+  const K key = i < n ? keys[i] : outside;
+  K prev = __shfl_up_sync(kFullMask, key, 1);
+  if (lane == 0 && w0 != 0) prev = keys[w0 - 1];
+  const bool valid = key < outside;
+  const bool start = valid && (i == 0 || prev != key);
+  uint64_t mask = valid ? mask_of(i) : 0ull;
+#pragma unroll
+  for (uint32_t d = 1; d < kWarp; d <<= 1) { // equal keys lie side by side
+    const uint64_t m = __shfl_down_sync(kFullMask, mask, d);
+    const K k = __shfl_down_sync(kFullMask, key, d);
+    if (lane + d < kWarp && k == key) mask |= m;
+  }
+  const uint32_t starts = __ballot_sync(kFullMask, start);
+  const K last = __shfl_sync(kFullMask, key, kWarp - 1);
+  const uint32_t owner = starts ? 31u - __clz(starts) : 0u;
+  if (starts && last < outside && __shfl_sync(kFullMask, key, owner) == last) {
+    uint64_t more = 0;
+    for (uint64_t j = w0 + kWarp; j < n; j += kWarp) {
+      const bool same = j + lane < n && keys[j + lane] == last;
+      if (same) more |= mask_of(j + lane);
+      if (!__all_sync(kFullMask, same)) break;
+    }
+    const uint32_t lo = __reduce_or_sync(kFullMask, static_cast<uint32_t>(more));
+    const uint32_t hi = __reduce_or_sync(kFullMask, static_cast<uint32_t>(more >> 32));
+    if (lane == owner) mask |= (static_cast<uint64_t>(hi) << 32) | lo;
+  }
   if (i >= n) return;
-  const uint64_t key = keys[i];
-  const bool valid = key < (1ull << (3 * depth));
-  const bool start = valid && (i == 0 || keys[i - 1] != key);
+  const uint32_t at = offsets[i];
   if (start) {
-    uint64_t mask = 0;
-    for (uint64_t j = i; j < n && keys[j] == key; ++j) {
-      if constexpr (Commands) {
-        const vx_leaf_command &c = cmds[bits[j]];
-        mask |= static_cast<uint64_t>(c.voxel_data_low) |
-                (static_cast<uint64_t>(c.voxel_data_high) << 32);
-      } else {
-        mask |= 1ull << bits[j];
-      }
-    }
-    uint32_t lx = 0, ly = 0, lz = 0;
-    for (uint32_t l = 0; l < depth; ++l) {
-      const uint32_t c = static_cast<uint32_t>(key >> (3 * (depth - 1 - l))) & 7u;
-      lx = (lx << 1) | (c & 1u);
-      ly = (ly << 1) | ((c >> 1) & 1u);
-      lz = (lz << 1) | ((c >> 2) & 1u);
-    }
     vx_primitive p{};
-    p.c[0] = static_cast<int32_t>(lx * 4);
-    p.c[1] = static_cast<int32_t>(ly * 4);
-    p.c[2] = static_cast<int32_t>(lz * 4);
+    p.c[0] = static_cast<int32_t>(compact3(key) * 4u);
+    p.c[1] = static_cast<int32_t>(compact3(key >> 1) * 4u);
+    p.c[2] = static_cast<int32_t>(compact3(key >> 2) * 4u);
     p.r[0] = static_cast<uint32_t>(mask);
     p.r[1] = static_cast<uint32_t>(mask >> 32);
     p.flags = vx_make_flags(kShapeLeafMask, op, material);
-    out[offsets[i]] = p;
+    out[at] = p;
+    leaf_keys[at] = key;
   }
-  if (i == n - 1) *out_count = offsets[i] + (start ? 1u : 0u);
+  if (i == n - 1) *out_count = at + (start ? 1u : 0u);
 }
 
 } // namespace vx::dag
@@ -793,16 +840,19 @@ vx_status run_pipeline(vx_dag *d, const vx_primitive *prims,
                        const uint32_t *d_count, uint32_t host_count,
                        cudaStream_t s, bool terrain = false,
                        uint32_t blocks_per_sm = 0 /* 0: the edit.blocks_per_sm knob */,
-                       int small = -1 /* -1: by host_count as a primitive batch */) {
+                       int small = -1 /* -1: by host_count as a primitive batch */,
+                       const uint64_t *sorted_keys = nullptr /* EditCtx::sorted_keys */) {
   Ctx x{d->t, d->a, prims, d_count, host_count};
-  const EditCtx e{d->t.hdr, d->a, prims, d_count, host_count, d->t.depth,
-                  static_cast<uint32_t>(tune::get(tune::kEditBigItem))};
+  EditCtx e{d->t.hdr, d->a, prims, d_count, host_count, d->t.depth,
+            static_cast<uint32_t>(tune::get(tune::kEditBigItem)), nullptr};
   const uint32_t depth = d->t.depth;
   const uint32_t grid = static_cast<uint32_t>(sm_count()) *
                         (blocks_per_sm ? blocks_per_sm
                                        : static_cast<uint32_t>(tune::get(tune::kEditBlocksPerSm)));
   if (!terrain && (small < 0 ? small_batch(host_count, false) : small != 0))
     return run_small(d, x, e, s);
+  e.sorted_keys = sorted_keys;
+  if (sorted_keys != nullptr) e.big_item = 0xffffffffu; // no list is walked
   {
     prof::Scope sc("dag_init", s);
     init_kernel<<<std::min<uint32_t>(grid, ceil_div(std::max(host_count, 1u), kBlock) + 1),
@@ -811,20 +861,26 @@ vx_status run_pipeline(vx_dag *d, const vx_primitive *prims,
   VX_TRY_CUDA(cudaGetLastError());
   DagTree tree{d->t};
   for (uint32_t l = 0; l + 1 < depth; ++l) {
+    const uint32_t lgrid = level_grid(grid, l, kBlock / 8);
     {
       prof::Scope sc("dag_expand", s);
       if (terrain)
-        expand_kernel<DagTree, true><<<grid, kBlock, 0, s>>>(e, tree, l);
+        expand_kernel<DagTree, true><<<lgrid, kBlock, 0, s>>>(e, tree, l);
+      else if (sorted_keys != nullptr)
+        expand_sorted_kernel<DagTree><<<lgrid, kBlock, 0, s>>>(e, tree, l);
       else
-        expand_kernel<DagTree, false><<<grid, kBlock, 0, s>>>(e, tree, l);
+        expand_kernel<DagTree, false><<<lgrid, kBlock, 0, s>>>(e, tree, l);
     }
     VX_TRY_CUDA(cudaGetLastError());
+    if (sorted_keys != nullptr) continue;
     {
       prof::Scope sc("dag_expand_big", s);
       if (terrain)
-        expand_big_kernel<DagTree, true><<<sm_count() * 2, kBlock, 0, s>>>(e, tree, l);
+        expand_big_kernel<DagTree, true>
+            <<<level_grid(sm_count() * 2, l, 1), kBlock, 0, s>>>(e, tree, l);
       else
-        expand_big_kernel<DagTree, false><<<sm_count(), kBigBlock, 0, s>>>(e, tree, l);
+        expand_big_kernel<DagTree, false>
+            <<<level_grid(sm_count(), l, 1), kBigBlock, 0, s>>>(e, tree, l);
     }
     VX_TRY_CUDA(cudaGetLastError());
   }
@@ -869,7 +925,7 @@ vx_status run_pipeline(vx_dag *d, const vx_primitive *prims,
   VX_TRY_CUDA(cudaGetLastError());
   for (uint32_t r = depth - 1; r > 0; --r) {
     prof::Scope sc("dag_build", s);
-    build_kernel<<<grid, kBlock, 0, s>>>(x, r - 1);
+    build_kernel<<<level_grid(grid, r - 1, kBlock), kBlock, 0, s>>>(x, r - 1);
     VX_TRY_CUDA(cudaGetLastError());
   }
   {
@@ -877,6 +933,13 @@ vx_status run_pipeline(vx_dag *d, const vx_primitive *prims,
     publish_kernel<<<1, 1, 0, s>>>(x);
   }
   return from_cuda(cudaGetLastError());
+}
+
+// A prepared list of `count` voxels or leaf commands: small ones in one
+// cooperative launch, the others level by level in key order.
+vx_status run_list(vx_dag *d, const vx::plain::Prepared &list, uint32_t count, cudaStream_t s) {
+  return run_pipeline(d, list.prims, list.count, count, s, false, 0, small_batch(count, true),
+                      list.leaf_keys);
 }
 
 // The device status, read through a pinned word (a copy into pageable
@@ -962,73 +1025,83 @@ size_t workspace_size(uint32_t count) {
   return c.offset;
 }
 
-// Voxel list -> one leaf-mask primitive per touched leaf (op, material),
-// written into the workspace; *out_prims / *out_count point into it.
-vx_status prepare(const vx_voxel *edits, uint32_t count, uint32_t depth,
-                  uint32_t op, uint32_t material, void *workspace,
-                  const vx_primitive **out_prims, const uint32_t **out_count,
-                  cudaStream_t s) {
+namespace {
+
+// Packed (leaf key, bit or command index) entries, sorted by key and reduced
+// to one leaf-mask primitive per leaf, in key order.
+template <class K, class Pack>
+vx_status prepare_keys(Pack pack, const vx_leaf_command *cmds, uint32_t count, uint32_t depth,
+                       uint32_t op, uint32_t material, void *workspace, Prepared *out,
+                       cudaStream_t s) {
   using namespace vx::dag;
   vx::Carver c(workspace);
   const PlainLayout p = plain_layout(c, count);
   const uint32_t blocks = vx::ceil_div(count, kBlock);
-  {
-    vx::prof::Scope sc("plain_pack_voxels", s);
-    pack_voxels_kernel<<<blocks, kBlock, 0, s>>>(edits, count, depth, p.keys, p.bits);
-  }
+  K *keys = reinterpret_cast<K *>(p.keys);
+  pack(keys, p.bits, blocks);
   VX_TRY_CUDA(cudaGetLastError());
-  VX_TRY(vx_sort_pairs_u64(p.keys, p.bits, count, 3 * depth + 1, p.sort_ws,
-                           p.sort_ws_bytes, s));
+  if constexpr (sizeof(K) == 4)
+    VX_TRY(vx_sort_pairs_u32(keys, p.bits, count, 3 * depth + 1, p.sort_ws, p.sort_ws_bytes, s));
+  else
+    VX_TRY(vx_sort_pairs_u64(keys, p.bits, count, 3 * depth + 1, p.sort_ws, p.sort_ws_bytes, s));
   {
     vx::prof::Scope sc("plain_run_flags", s);
-    run_flags_kernel<<<blocks, kBlock, 0, s>>>(p.keys, count, depth, p.offsets);
+    run_flags_kernel<K><<<blocks, kBlock, 0, s>>>(keys, count, depth, p.offsets);
   }
   VX_TRY_CUDA(cudaGetLastError());
   VX_TRY(vx_scan_exclusive_sum_u32(p.offsets, count, p.scan_ws, p.scan_ws_bytes, s));
+  // The leaves' keys take the place of the sort's scratch (which holds a copy
+  // of the 64-bit keys); a list of one entry sorts without scratch, and its
+  // own word is read before its leaf's key replaces it.
+  uint64_t *leaf_keys = count > 1 ? static_cast<uint64_t *>(p.sort_ws) : p.keys;
   {
     vx::prof::Scope sc("plain_reduce_runs", s);
-    reduce_runs_kernel<false><<<blocks, kBlock, 0, s>>>(p.keys, p.bits, nullptr, p.offsets,
-                                                        count, depth, op, material, p.prims,
-                                                        p.count);
+    if (cmds != nullptr)
+      reduce_runs_kernel<K, true><<<blocks, kBlock, 0, s>>>(keys, p.bits, cmds, p.offsets, count,
+                                                            depth, op, material, p.prims,
+                                                            leaf_keys, p.count);
+    else
+      reduce_runs_kernel<K, false><<<blocks, kBlock, 0, s>>>(keys, p.bits, nullptr, p.offsets,
+                                                             count, depth, op, material, p.prims,
+                                                             leaf_keys, p.count);
   }
   VX_TRY_CUDA(cudaGetLastError());
-  *out_prims = p.prims;
-  *out_count = p.count;
+  *out = Prepared{p.prims, p.count, leaf_keys};
   return VX_OK;
+}
+
+} // namespace
+
+// Voxel list -> one leaf-mask primitive per touched leaf (op, material),
+// written into the workspace.
+vx_status prepare(const vx_voxel *edits, uint32_t count, uint32_t depth,
+                  uint32_t op, uint32_t material, void *workspace, Prepared *out,
+                  cudaStream_t s) {
+  using namespace vx::dag;
+  auto pack = [&](auto *keys, uint32_t *bits, uint32_t blocks) {
+    using K = std::remove_pointer_t<decltype(keys)>;
+    vx::prof::Scope sc("plain_pack_voxels", s);
+    pack_voxels_kernel<K><<<blocks, kBlock, 0, s>>>(edits, count, depth, keys, bits);
+  };
+  return depth <= kMaxDepthKey32
+             ? prepare_keys<uint32_t>(pack, nullptr, count, depth, op, material, workspace, out, s)
+             : prepare_keys<uint64_t>(pack, nullptr, count, depth, op, material, workspace, out, s);
 }
 
 // Leaf edit commands -> one leaf-mask primitive per named leaf, the masks of
 // commands naming the same leaf OR-merged (the engine's merge_commands).
 vx_status prepare_leaf_commands(const vx_leaf_command *cmds, uint32_t count, uint32_t depth,
-                                uint32_t op, uint32_t material, void *workspace,
-                                const vx_primitive **out_prims, const uint32_t **out_count,
+                                uint32_t op, uint32_t material, void *workspace, Prepared *out,
                                 cudaStream_t s) {
   using namespace vx::dag;
-  vx::Carver c(workspace);
-  const PlainLayout p = plain_layout(c, count);
-  const uint32_t blocks = vx::ceil_div(count, kBlock);
-  {
+  auto pack = [&](auto *keys, uint32_t *index, uint32_t blocks) {
+    using K = std::remove_pointer_t<decltype(keys)>;
     vx::prof::Scope sc("plain_pack_leaf_commands", s);
-    pack_leaf_commands_kernel<<<blocks, kBlock, 0, s>>>(cmds, count, depth, p.keys, p.bits);
-  }
-  VX_TRY_CUDA(cudaGetLastError());
-  VX_TRY(vx_sort_pairs_u64(p.keys, p.bits, count, 3 * depth + 1, p.sort_ws,
-                           p.sort_ws_bytes, s));
-  {
-    vx::prof::Scope sc("plain_run_flags", s);
-    run_flags_kernel<<<blocks, kBlock, 0, s>>>(p.keys, count, depth, p.offsets);
-  }
-  VX_TRY_CUDA(cudaGetLastError());
-  VX_TRY(vx_scan_exclusive_sum_u32(p.offsets, count, p.scan_ws, p.scan_ws_bytes, s));
-  {
-    vx::prof::Scope sc("plain_reduce_runs", s);
-    reduce_runs_kernel<true><<<blocks, kBlock, 0, s>>>(p.keys, p.bits, cmds, p.offsets, count,
-                                                       depth, op, material, p.prims, p.count);
-  }
-  VX_TRY_CUDA(cudaGetLastError());
-  *out_prims = p.prims;
-  *out_count = p.count;
-  return VX_OK;
+    pack_leaf_commands_kernel<K><<<blocks, kBlock, 0, s>>>(cmds, count, depth, keys, index);
+  };
+  return depth <= kMaxDepthKey32
+             ? prepare_keys<uint32_t>(pack, cmds, count, depth, op, material, workspace, out, s)
+             : prepare_keys<uint64_t>(pack, cmds, count, depth, op, material, workspace, out, s);
 }
 
 } // namespace vx::plain
@@ -1157,7 +1230,7 @@ vx_status vx_dag_apply_voxels(vx_dag *d, const vx_voxel *edits, uint32_t count,
     // one cooperative launch: voxels -> leaf masks -> the edit
     Ctx x{d->t, d->a, prep.prims, prep.nprims, count};
     const EditCtx e{d->t.hdr, d->a, prep.prims, prep.nprims, count, d->t.depth,
-                    static_cast<uint32_t>(vx::tune::get(vx::tune::kEditBigItem))};
+                    static_cast<uint32_t>(vx::tune::get(vx::tune::kEditBigItem)), nullptr};
     if (d->status_alias == nullptr) {
       VX_TRY(run_small(d, x, e, s, &prep));
       return read_status(d, s, true);
@@ -1166,10 +1239,9 @@ vx_status vx_dag_apply_voxels(vx_dag *d, const vx_voxel *edits, uint32_t count,
     VX_TRY(run_small(d, x, e, s, &prep, d->status_alias));
     return read_written_status(d, s);
   }
-  const vx_primitive *prims = nullptr;
-  const uint32_t *n = nullptr;
-  VX_TRY(vx::plain::prepare(edits, count, d->t.depth, op, 0, workspace, &prims, &n, s));
-  VX_TRY(run_pipeline(d, prims, n, count, s, false, 0, small_batch(count, true)));
+  vx::plain::Prepared list;
+  VX_TRY(vx::plain::prepare(edits, count, d->t.depth, op, 0, workspace, &list, s));
+  VX_TRY(run_list(d, list, count, s));
   return read_status(d, s, true);
 }
 
@@ -1183,11 +1255,9 @@ vx_status vx_dag_apply_leaf_commands(vx_dag *d, const vx_leaf_command *cmds, uin
   if (workspace == nullptr || workspace_bytes < vx_leaf_command_workspace_size(count))
     return VX_ERR_INVALID_VALUE;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const vx_primitive *prims = nullptr;
-  const uint32_t *n = nullptr;
-  VX_TRY(vx::plain::prepare_leaf_commands(cmds, count, d->t.depth, op, 0, workspace, &prims, &n,
-                                          s));
-  VX_TRY(run_pipeline(d, prims, n, count, s, false, 0, small_batch(count, true)));
+  vx::plain::Prepared list;
+  VX_TRY(vx::plain::prepare_leaf_commands(cmds, count, d->t.depth, op, 0, workspace, &list, s));
+  VX_TRY(run_list(d, list, count, s));
   return read_status(d, s, true);
 }
 
@@ -1232,10 +1302,9 @@ vx_status vx_dag_graph_voxels(vx_dag *d, const vx_voxel *edits, uint32_t count, 
     return VX_ERR_INVALID_VALUE;
   return vx::graph::capture(
       [&](cudaStream_t s) {
-        const vx_primitive *prims = nullptr;
-        const uint32_t *n = nullptr;
-        VX_TRY(vx::plain::prepare(edits, count, d->t.depth, op, 0, workspace, &prims, &n, s));
-        return run_pipeline(d, prims, n, count, s, false, 0, small_batch(count, true));
+        vx::plain::Prepared list;
+        VX_TRY(vx::plain::prepare(edits, count, d->t.depth, op, 0, workspace, &list, s));
+        return run_list(d, list, count, s);
       },
       out);
 }

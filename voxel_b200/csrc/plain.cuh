@@ -8,12 +8,19 @@
 
 namespace vx::plain {
 size_t workspace_size(uint32_t count);
+
+// The leaf-mask primitives a list became, in the caller's workspace: in
+// ascending order of their leaf keys (3 bits per inner level, the root's child
+// highest), one per touched leaf.
+struct Prepared {
+  const vx_primitive *prims;
+  const uint32_t *count;      // device count of them
+  const uint64_t *leaf_keys;
+};
 vx_status prepare(const vx_voxel *edits, uint32_t count, uint32_t depth,
                   uint32_t op, uint32_t material, void *workspace,
-                  const vx_primitive **out_prims, const uint32_t **out_count,
-                  cudaStream_t s);
+                  Prepared *out, cudaStream_t s);
 vx_status prepare_leaf_commands(const vx_leaf_command *cmds, uint32_t count, uint32_t depth,
                                 uint32_t op, uint32_t material, void *workspace,
-                                const vx_primitive **out_prims, const uint32_t **out_count,
-                                cudaStream_t s);
+                                Prepared *out, cudaStream_t s);
 } // namespace vx::plain

@@ -702,16 +702,19 @@ vx_status launch_collection(const Tables &t, uint32_t grid, cudaStream_t s, bool
 
 vx_status run_pipeline(vx_svo *v, const vx_primitive *prims, const uint32_t *d_count,
                        uint32_t host_count, cudaStream_t s, bool terrain,
-                       int small = -1 /* -1: by host_count as a primitive batch */) {
+                       int small = -1 /* -1: by host_count as a primitive batch */,
+                       const uint64_t *sorted_keys = nullptr /* EditCtx::sorted_keys */) {
   const Tables &t = v->t;
-  const EditCtx e{t.hdr, v->a, prims, d_count, host_count, t.depth,
-                  static_cast<uint32_t>(tune::get(tune::kEditBigItem))};
+  EditCtx e{t.hdr, v->a, prims, d_count, host_count, t.depth,
+            static_cast<uint32_t>(tune::get(tune::kEditBigItem)), nullptr};
   const SvoTree pol{t};
   const uint32_t depth = t.depth;
   const uint32_t grid = static_cast<uint32_t>(sm_count()) *
                         static_cast<uint32_t>(tune::get(tune::kEditBlocksPerSm));
   if (!terrain && (small < 0 ? small_batch(host_count, false) : small != 0))
     return run_small(e, t, s);
+  e.sorted_keys = sorted_keys;
+  if (sorted_keys != nullptr) e.big_item = 0xffffffffu; // no list is walked
   {
     prof::Scope sc("svo_init", s);
     begin_kernel<<<1, 1, 0, s>>>(t);
@@ -720,16 +723,23 @@ vx_status run_pipeline(vx_svo *v, const vx_primitive *prims, const uint32_t *d_c
   }
   VX_TRY_CUDA(cudaGetLastError());
   for (uint32_t l = 0; l + 1 < depth; ++l) {
+    const uint32_t lgrid = level_grid(grid, l, kBlock / 8);
     {
       prof::Scope sc("svo_expand", s);
-      if (terrain) expand_kernel<SvoTree, true><<<grid, kBlock, 0, s>>>(e, pol, l);
-      else expand_kernel<SvoTree, false><<<grid, kBlock, 0, s>>>(e, pol, l);
+      if (terrain) expand_kernel<SvoTree, true><<<lgrid, kBlock, 0, s>>>(e, pol, l);
+      else if (sorted_keys) expand_sorted_kernel<SvoTree><<<lgrid, kBlock, 0, s>>>(e, pol, l);
+      else expand_kernel<SvoTree, false><<<lgrid, kBlock, 0, s>>>(e, pol, l);
     }
     VX_TRY_CUDA(cudaGetLastError());
+    if (sorted_keys != nullptr) continue;
     {
       prof::Scope sc("svo_expand_big", s);
-      if (terrain) expand_big_kernel<SvoTree, true><<<sm_count() * 2, kBlock, 0, s>>>(e, pol, l);
-      else expand_big_kernel<SvoTree, false><<<sm_count(), kBigBlock, 0, s>>>(e, pol, l);
+      if (terrain)
+        expand_big_kernel<SvoTree, true>
+            <<<level_grid(sm_count() * 2, l, 1), kBlock, 0, s>>>(e, pol, l);
+      else
+        expand_big_kernel<SvoTree, false>
+            <<<level_grid(sm_count(), l, 1), kBigBlock, 0, s>>>(e, pol, l);
     }
     VX_TRY_CUDA(cudaGetLastError());
   }
@@ -746,7 +756,7 @@ vx_status run_pipeline(vx_svo *v, const vx_primitive *prims, const uint32_t *d_c
   VX_TRY_CUDA(cudaGetLastError());
   for (uint32_t r = depth - 1; r > 0; --r) {
     prof::Scope sc("svo_build", s);
-    build_kernel<<<grid, kBlock, 0, s>>>(e, t, r - 1);
+    build_kernel<<<level_grid(grid, r - 1, kBlock), kBlock, 0, s>>>(e, t, r - 1);
     VX_TRY_CUDA(cudaGetLastError());
   }
   {
@@ -754,6 +764,13 @@ vx_status run_pipeline(vx_svo *v, const vx_primitive *prims, const uint32_t *d_c
     finalize_kernel<<<1, 1, 0, s>>>(t);
   }
   return from_cuda(cudaGetLastError());
+}
+
+// A prepared list of `count` voxels or leaf commands: small ones in one
+// cooperative launch, the others level by level in key order.
+vx_status run_list(vx_svo *v, const vx::plain::Prepared &list, uint32_t count, cudaStream_t s) {
+  return run_pipeline(v, list.prims, list.count, count, s, false, small_batch(count, true),
+                      list.leaf_keys);
 }
 
 // The device status, read through a pinned word (a copy into pageable
@@ -911,15 +928,13 @@ vx_status vx_svo_apply_voxels(vx_svo *v, const vx_voxel *edits, uint32_t count,
   if (workspace == nullptr || workspace_bytes < vx_svo_voxel_workspace_size(count))
     return VX_ERR_INVALID_VALUE;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const vx_primitive *prims = nullptr;
-  const uint32_t *n = nullptr;
   const uint32_t mat = op == VX_EDIT_PLACE ? (material ? material : 1u) : 0u;
   PlainPrep prep;
   if (small_batch(count, true) &&
       plain_prep_layout(workspace, workspace_bytes, edits, count, op, mat, &prep)) {
     // one cooperative launch: voxels -> leaf masks -> the edit and collection
     const EditCtx e{v->t.hdr, v->a, prep.prims, prep.nprims, count, v->t.depth,
-                    static_cast<uint32_t>(vx::tune::get(vx::tune::kEditBigItem))};
+                    static_cast<uint32_t>(vx::tune::get(vx::tune::kEditBigItem)), nullptr};
     if (v->status_alias == nullptr) {
       VX_TRY(run_small(e, v->t, s, &prep));
       return read_status(v, s);
@@ -928,8 +943,9 @@ vx_status vx_svo_apply_voxels(vx_svo *v, const vx_voxel *edits, uint32_t count,
     VX_TRY(run_small(e, v->t, s, &prep, v->status_alias));
     return read_written_status(v, s);
   }
-  VX_TRY(vx::plain::prepare(edits, count, v->t.depth, op, mat, workspace, &prims, &n, s));
-  VX_TRY(run_pipeline(v, prims, n, count, s, false, small_batch(count, true)));
+  vx::plain::Prepared list;
+  VX_TRY(vx::plain::prepare(edits, count, v->t.depth, op, mat, workspace, &list, s));
+  VX_TRY(run_list(v, list, count, s));
   return read_status(v, s);
 }
 
@@ -942,12 +958,10 @@ vx_status vx_svo_apply_leaf_commands(vx_svo *v, const vx_leaf_command *cmds, uin
   if (workspace == nullptr || workspace_bytes < vx_leaf_command_workspace_size(count))
     return VX_ERR_INVALID_VALUE;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const vx_primitive *prims = nullptr;
-  const uint32_t *n = nullptr;
   const uint32_t mat = op == VX_EDIT_PLACE ? (material ? material : 1u) : 0u;
-  VX_TRY(vx::plain::prepare_leaf_commands(cmds, count, v->t.depth, op, mat, workspace, &prims,
-                                          &n, s));
-  VX_TRY(run_pipeline(v, prims, n, count, s, false, small_batch(count, true)));
+  vx::plain::Prepared list;
+  VX_TRY(vx::plain::prepare_leaf_commands(cmds, count, v->t.depth, op, mat, workspace, &list, s));
+  VX_TRY(run_list(v, list, count, s));
   return read_status(v, s);
 }
 
