@@ -179,16 +179,11 @@ __device__ __forceinline__ bool edit_fits(const Tables &t) {
 // edit has only read the tree so far, so marking from the current root
 // keeps everything it reads).  A capacity error follows only if the edit
 // still does not fit after it.
-__device__ __forceinline__ void check_capacity_body(Tables t) {
-  Header *h = t.hdr;
-  t.ctr->gc_needed = 0;
-  if (h->status != kDevOk) return;
-  if (!edit_fits(t)) {
-    if (t.ctr->detached) t.ctr->gc_needed = 1;
-    else h->status = kDevCapacity;
-  }
+__device__ __forceinline__ uint32_t capacity_verdict(const Tables &t) {
+  // 0 fits (or the edit has failed already), 1 collect first, 2 no room
+  if (t.hdr->status != kDevOk || edit_fits(t)) return 0u;
+  return t.ctr->detached ? 1u : 2u;
 }
-__global__ void check_capacity_kernel(Tables t) { check_capacity_body(t); }
 
 __device__ void finish_upwards(const EditCtx &x, const Tables &t, uint32_t parent, uint32_t l);
 
@@ -442,42 +437,69 @@ __global__ void finalize_kernel(Tables t) { finalize_body(t); }
 
 // ------------------------------------------------------------------- GC --
 
+// Sixteen marks per store (cudaMalloc aligns the arrays to 256 bytes).
+__device__ __forceinline__ void clear_marks(uint8_t *m, uint32_t n, Blocks blk) {
+  const uint64_t first = blk.id * static_cast<uint64_t>(blockDim.x) + threadIdx.x;
+  const uint64_t stride = static_cast<uint64_t>(blk.count) * blockDim.x;
+  for (uint64_t i = first; i < n / 16u; i += stride)
+    reinterpret_cast<uint4 *>(m)[i] = make_uint4(0u, 0u, 0u, 0u);
+  if (first < n % 16u) m[n - 1u - first] = 0;
+}
+
 __device__ __forceinline__ void gc_clear_body(Tables t, Blocks blk) {
   Counters *c = t.ctr;
   if (!c->gc_needed) return;
-  for (uint64_t i = blk.id * static_cast<uint64_t>(blockDim.x) + threadIdx.x;
-       i < c->node_count; i += static_cast<uint64_t>(blk.count) * blockDim.x)
-    t.node_mark[i] = 0;
-  for (uint64_t i = blk.id * static_cast<uint64_t>(blockDim.x) + threadIdx.x;
-       i < c->leaf_count; i += static_cast<uint64_t>(blk.count) * blockDim.x)
-    t.leaf_mark[i] = 0;
+  clear_marks(t.node_mark, c->node_count, blk);
+  clear_marks(t.leaf_mark, c->leaf_count, blk);
   if (blk.id == 0 && threadIdx.x == 0) {
     for (uint32_t l = 0; l <= kMaxDepth; ++l) c->gc_count[l] = 0;
     c->gc_count[0] = 1;
     t.front[0][0] = 0; // the root
   }
 }
-__global__ void gc_clear_kernel(Tables t) { gc_clear_body(t, launch_blocks()); }
 
+// Marks level l's nodes and lists their child nodes for level l + 1: a lane
+// reads a node's 8 words by two loads, and a warp takes room for all its
+// lanes' children with one atomic (the level's counter is one address).
 __device__ __forceinline__ void gc_level_body(Tables t, uint32_t l, Blocks blk) {
   Counters *c = t.ctr;
   if (!c->gc_needed) return;
   const uint32_t n = c->gc_count[l];
   const uint32_t *front = t.front[l & 1u];
   uint32_t *next = t.front[(l + 1) & 1u];
-  for (uint64_t i = blk.id * static_cast<uint64_t>(blockDim.x) + threadIdx.x; i < n;
-       i += static_cast<uint64_t>(blk.count) * blockDim.x) {
-    const uint32_t node = front[i];
-    t.node_mark[node] = 1;
-    for (uint32_t k = 0; k < 8; ++k) {
-      const uint32_t w = t.nodes[static_cast<size_t>(node) * 8u + k];
-      if (!(w & kChild)) continue;
-      if (l + 1 < t.depth) next[atomicAdd(&c->gc_count[l + 1], 1u)] = w & kIndex;
-      else t.leaf_mark[w & kIndex] = 1;
+  const bool inner = l + 1 < t.depth;
+  const uint32_t lane = lane_id();
+  const uint64_t stride = static_cast<uint64_t>(blk.count) * blockDim.x;
+  for (uint64_t g = blk.id * static_cast<uint64_t>(blockDim.x) + threadIdx.x - lane; g < n;
+       g += stride) {
+    const uint64_t i = g + lane;
+    uint32_t w[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    if (i < n) {
+      const uint32_t node = front[i];
+      t.node_mark[node] = 1;
+      const uint4 *src = reinterpret_cast<const uint4 *>(t.nodes + static_cast<size_t>(node) * 8u);
+      const uint4 a = src[0], b = src[1];
+      w[0] = a.x; w[1] = a.y; w[2] = a.z; w[3] = a.w;
+      w[4] = b.x; w[5] = b.y; w[6] = b.z; w[7] = b.w;
     }
+    if (!inner) {
+#pragma unroll
+      for (uint32_t k = 0; k < 8; ++k)
+        if (w[k] & kChild) t.leaf_mark[w[k] & kIndex] = 1;
+      continue;
+    }
+    uint32_t count = 0;
+#pragma unroll
+    for (uint32_t k = 0; k < 8; ++k) count += (w[k] & kChild) ? 1u : 0u;
+    const uint32_t inc = warp_inclusive_sum(count);
+    uint32_t at = 0;
+    if (lane == kWarp - 1 && inc != 0) at = atomicAdd(&c->gc_count[l + 1], inc);
+    at = __shfl_sync(kFullMask, at, kWarp - 1) + inc - count;
+#pragma unroll
+    for (uint32_t k = 0; k < 8; ++k)
+      if (w[k] & kChild) next[at++] = w[k] & kIndex;
   }
 }
-__global__ void gc_level_kernel(Tables t, uint32_t l) { gc_level_body(t, l, launch_blocks()); }
 
 __device__ __forceinline__ void gc_zero_free_body(Tables t) {
   Counters *c = t.ctr;
@@ -485,20 +507,44 @@ __device__ __forceinline__ void gc_zero_free_body(Tables t) {
   c->free_node_count = 0;
   c->free_leaf_count = 0;
 }
-__global__ void gc_zero_free_kernel(Tables t) { gc_zero_free_body(t); }
+
+// Lists the unmarked slots from `first` on: four marks per lane and load, one
+// atomic per warp.
+__device__ __forceinline__ void list_unmarked(const uint8_t *mark, uint32_t first, uint32_t n,
+                                              uint32_t *list, uint32_t *count, Blocks blk) {
+  const uint32_t lane = lane_id();
+  const uint64_t stride = static_cast<uint64_t>(blk.count) * blockDim.x * 4u;
+  for (uint64_t g = (blk.id * static_cast<uint64_t>(blockDim.x) + threadIdx.x - lane) * 4u; g < n;
+       g += stride) {
+    const uint64_t i = g + lane * 4u;
+    uint32_t m = 0x01010101u; // marked: nothing to list
+    if (i + 4u <= n) {
+      m = *reinterpret_cast<const uint32_t *>(mark + i);
+    } else {
+      for (uint32_t k = 0; k < 4u && i + k < n; ++k)
+        if (!mark[i + k]) m &= ~(0xffu << (8u * k));
+    }
+    uint32_t free4 = 0;
+#pragma unroll
+    for (uint32_t k = 0; k < 4u; ++k)
+      if (((m >> (8u * k)) & 0xffu) == 0u && i + k >= first) free4 |= 1u << k;
+    const uint32_t inc = warp_inclusive_sum(static_cast<uint32_t>(__popc(free4)));
+    uint32_t at = 0;
+    if (lane == kWarp - 1 && inc != 0) at = atomicAdd(count, inc);
+    at = __shfl_sync(kFullMask, at, kWarp - 1) + inc - __popc(free4);
+#pragma unroll
+    for (uint32_t k = 0; k < 4u; ++k)
+      if (free4 & (1u << k)) list[at++] = static_cast<uint32_t>(i + k);
+  }
+}
 
 __device__ __forceinline__ void gc_rebuild_body(Tables t, Blocks blk) {
   Counters *c = t.ctr;
   if (!c->gc_needed) return;
-  const uint32_t nn = c->node_count, nl = c->leaf_count;
-  for (uint64_t i = 1 + blk.id * static_cast<uint64_t>(blockDim.x) + threadIdx.x; i < nn;
-       i += static_cast<uint64_t>(blk.count) * blockDim.x)
-    if (!t.node_mark[i]) t.free_nodes[atomicAdd(&c->free_node_count, 1u)] = static_cast<uint32_t>(i);
-  for (uint64_t i = blk.id * static_cast<uint64_t>(blockDim.x) + threadIdx.x; i < nl;
-       i += static_cast<uint64_t>(blk.count) * blockDim.x)
-    if (!t.leaf_mark[i]) t.free_leaves[atomicAdd(&c->free_leaf_count, 1u)] = static_cast<uint32_t>(i);
+  list_unmarked(t.node_mark, 1u /* the root stays */, c->node_count, t.free_nodes,
+                &c->free_node_count, blk);
+  list_unmarked(t.leaf_mark, 0u, c->leaf_count, t.free_leaves, &c->free_leaf_count, blk);
 }
-__global__ void gc_rebuild_kernel(Tables t) { gc_rebuild_body(t, launch_blocks()); }
 
 // After a collection inside an edit: the free lists are the edit's starting
 // point; the edit fails only if it still does not fit.
@@ -511,13 +557,54 @@ __device__ __forceinline__ void gc_recheck_body(Tables t) {
   c->base_free_leaves = c->free_leaf_count;
   if (t.hdr->status == kDevOk && !edit_fits(t)) t.hdr->status = kDevCapacity;
 }
-__global__ void gc_recheck_kernel(Tables t) { gc_recheck_body(t); }
 
-// vx_svo_collect: a collection on request, between edits.
-__global__ void gc_request_kernel(Tables t) { t.ctr->gc_needed = t.ctr->detached; }
-__global__ void gc_end_kernel(Tables t) {
-  if (t.ctr->gc_needed) t.ctr->detached = 0;
-  t.ctr->gc_needed = 0;
+// The collection's stages with grid-wide barriers between them; every block
+// of a cooperative launch calls it.
+__device__ __forceinline__ void collect_stages(const Tables &t, cooperative_groups::grid_group &grid,
+                                               Blocks blk, bool lead) {
+  if (lead) t.ctr->gc_needed = 1; // no block reads it before the barrier
+  grid.sync();
+  gc_clear_body(t, blk);
+  grid.sync();
+  for (uint32_t l = 0; l < t.depth; ++l) {
+    gc_level_body(t, l, blk);
+    grid.sync();
+  }
+  if (lead) gc_zero_free_body(t);
+  grid.sync();
+  gc_rebuild_body(t, blk);
+  grid.sync();
+}
+
+// The capacity check of the level-by-level pipeline with the collection it
+// may call for, or (on_request, vx_svo_collect) a collection between edits:
+// one cooperative launch whose blocks all reach the same verdict from counts
+// that are final, so the usual case (no collection) ends there.  As separate
+// kernels the stages took 14 launches that found nothing to do, 0.2 ms of a
+// batched edit of 32,768 primitives on B200.
+__global__ void __launch_bounds__(kBlock) collect_kernel(Tables t, bool on_request) {
+  cooperative_groups::grid_group grid = cooperative_groups::this_grid();
+  const Blocks blk = launch_blocks();
+  const bool lead = blk.id == 0 && threadIdx.x == 0;
+  __shared__ uint32_t s_verdict;
+  if (threadIdx.x == 0)
+    s_verdict = on_request ? (t.ctr->detached ? 1u : 0u) : capacity_verdict(t);
+  __syncthreads();
+  if (s_verdict != 1u) {
+    // (a block that reads the status after this write sees a failed edit and
+    // leaves too)
+    if (s_verdict == 2u && lead) t.hdr->status = kDevCapacity;
+    if (lead) t.ctr->gc_needed = 0;
+    return;
+  }
+  collect_stages(t, grid, blk, lead);
+  if (!lead) return;
+  if (on_request) {
+    t.ctr->detached = 0;
+    t.ctr->gc_needed = 0;
+  } else {
+    gc_recheck_body(t);
+  }
 }
 
 // A whole edit, collection included, in one cooperative launch: the stages
@@ -561,29 +648,14 @@ __global__ void __maxnreg__(255) small_edit_kernel(EditCtx e, Tables t, PlainPre
                                                           Blocks{blk.count - 1u - blk.id, blk.count});
     grid.sync();
   }
-  // Every block reaches the capacity verdict of check_capacity_body from the
+  // Every block reaches the capacity verdict from the
   // same final counts, so the common case (the edit fits) needs no barrier.
-  __shared__ uint32_t s_verdict; // 0 fits, 1 collect first, 2 no room
-  if (threadIdx.x == 0) {
-    uint32_t v = 0;
-    if (t.hdr->status == kDevOk && !edit_fits(t)) v = t.ctr->detached ? 1u : 2u;
-    s_verdict = v;
-  }
+  __shared__ uint32_t s_verdict;
+  if (threadIdx.x == 0) s_verdict = capacity_verdict(t);
   __syncthreads();
   const uint32_t verdict = s_verdict;
-  if (lead) t.ctr->gc_needed = verdict == 1u; // no other block reads it before a barrier
   if (verdict == 1u) {
-    grid.sync(); // gc_needed, read by every collection stage
-    gc_clear_body(t, blk);
-    grid.sync();
-    for (uint32_t l = 0; l < t.depth; ++l) {
-      gc_level_body(t, l, blk);
-      grid.sync();
-    }
-    if (lead) gc_zero_free_body(t);
-    grid.sync();
-    gc_rebuild_body(t, blk);
-    grid.sync();
+    collect_stages(t, grid, blk, lead);
     if (lead) gc_recheck_body(t);
     grid.sync();
   }
@@ -685,19 +757,28 @@ inline bool small_batch(uint32_t n, bool voxel_list) {
                                                          : tune::kEditSmallMaxPrims));
 }
 
-// The collection stages as kernels, each leaving at once unless gc_needed is
-// set: by the capacity check inside an edit (ended by gc_recheck_kernel), or
-// by gc_request_kernel when a caller asks (ended by gc_end_kernel).
-vx_status launch_collection(const Tables &t, uint32_t grid, cudaStream_t s, bool on_request) {
+// collect_kernel on as many blocks as are resident at once (queried once, at
+// SVO creation, so never first inside a stream capture), at most eight per SM.
+int g_collect_resident = -1;
+vx_status query_collect_residency() {
+  if (g_collect_resident >= 0) return VX_OK;
+  int n = 0;
+  VX_TRY_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+      &n, reinterpret_cast<const void *>(&collect_kernel), kBlock, 0));
+  g_collect_resident = n;
+  return VX_OK;
+}
+vx_status launch_collection(const Tables &t, cudaStream_t s, bool on_request) {
+  VX_TRY(query_collect_residency());
+  if (g_collect_resident < 1) return VX_ERR_INVALID_VALUE;
+  const uint32_t grid = static_cast<uint32_t>(sm_count()) *
+                        static_cast<uint32_t>(std::min(g_collect_resident, 8));
+  Tables tc = t;
+  void *args[] = {&tc, &on_request};
   prof::Scope sc("svo_gc", s);
-  if (on_request) gc_request_kernel<<<1, 1, 0, s>>>(t);
-  gc_clear_kernel<<<grid, kBlock, 0, s>>>(t);
-  for (uint32_t l = 0; l < t.depth; ++l) gc_level_kernel<<<grid, kBlock, 0, s>>>(t, l);
-  gc_zero_free_kernel<<<1, 1, 0, s>>>(t);
-  gc_rebuild_kernel<<<grid, kBlock, 0, s>>>(t);
-  if (on_request) gc_end_kernel<<<1, 1, 0, s>>>(t);
-  else gc_recheck_kernel<<<1, 1, 0, s>>>(t);
-  return from_cuda(cudaGetLastError());
+  VX_TRY_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(&collect_kernel),
+                                          dim3(grid), dim3(kBlock), args, 0, s));
+  return VX_OK;
 }
 
 vx_status run_pipeline(vx_svo *v, const vx_primitive *prims, const uint32_t *d_count,
@@ -743,11 +824,7 @@ vx_status run_pipeline(vx_svo *v, const vx_primitive *prims, const uint32_t *d_c
     }
     VX_TRY_CUDA(cudaGetLastError());
   }
-  {
-    prof::Scope sc("svo_check_capacity", s);
-    check_capacity_kernel<<<1, 1, 0, s>>>(t);
-  }
-  VX_TRY(launch_collection(t, grid, s, false));
+  VX_TRY(launch_collection(t, s, false));
   {
     prof::Scope sc("svo_leafparent", s);
     if (terrain) leafparent_kernel<true><<<grid, kBlock, 0, s>>>(e, t);
@@ -835,7 +912,9 @@ vx_status vx_svo_create(const vx_svo_config *cfg, vx_svo **out) {
     return vx::from_cuda(e);
   };
   cudaError_t e;
-  if (vx_status qs = vx::svo::query_small_residency(); qs != VX_OK) {
+  vx_status qs = vx::svo::query_small_residency();
+  if (qs == VX_OK) qs = vx::svo::query_collect_residency();
+  if (qs != VX_OK) {
     vx_svo_destroy(v);
     return qs;
   }
@@ -1024,9 +1103,7 @@ vx_status vx_svo_query(const vx_svo *v, const vx_voxel *pts, uint32_t count,
 
 vx_status vx_svo_collect(vx_svo *v, vx_stream stream) {
   if (v == nullptr) return VX_ERR_INVALID_VALUE;
-  const uint32_t grid = static_cast<uint32_t>(vx::sm_count()) *
-                        static_cast<uint32_t>(vx::tune::get(vx::tune::kEditBlocksPerSm));
-  return launch_collection(v->t, grid, static_cast<cudaStream_t>(stream), true);
+  return launch_collection(v->t, static_cast<cudaStream_t>(stream), true);
 }
 
 vx_status vx_svo_get_counters(const vx_svo *v, vx_svo_counters *host, vx_stream stream) {
