@@ -295,24 +295,17 @@ __global__ void mark_pools_kernel(Tables t) {
   if (threadIdx.x < kMaxDepth) t.hdr->pool_mark[threadIdx.x] = t.hdr->pool_used[threadIdx.x];
 }
 
-// Level depth - 1: evaluate the 8 leaves of every item and hash-cons the
-// item.  Lanes (the tuning knob "edit.leafparent_lanes") threads share an
-// item, each evaluating children q + Lanes * j of it (q its rank in the
-// group): 8 lanes take one leaf each, 4 lanes two, which halves the
-// per-item work that every lane repeats and doubles the items in flight.
-// MinBlocks (the knob "edit.leafparent_blocks") trades registers for
-// resident blocks: the kernel is bound by chains of dependent loads, so more
-// items in flight can outweigh a few spilled values.
+// Level depth - 1 of a terrain build and of the small cooperative edits:
+// evaluate the 8 leaves of every item and hash-cons the item.  Lanes (the
+// tuning knob "edit.leafparent_lanes") threads share an item, each evaluating
+// children q + Lanes * j of it (q its rank in the group): a small edit has
+// fewer items than the chip has lanes, so an item's leaves are spread.
+// Batches take leafparent_kernel below.
 __device__ void finish_upwards(const Ctx &x, uint32_t parent, uint32_t l);
 
 // Climb: after storing an item's result, finish its ancestors (the single
 // cooperative kernel's bottom-up build, without level barriers).
-// Prefetch (the knob "edit.leafparent_prefetch"): beside each item's record,
-// load the old ref of the group's next item, and once the current item's old
-// leaves are requested, prefetch that next old node into L2, so the next
-// iteration's first dependent read (node header and child refs) is an L2 hit
-// instead of a DRAM round trip.
-template <bool Terrain, uint32_t Lanes, bool Climb = false, bool Prefetch = false>
+template <bool Terrain, uint32_t Lanes, bool Climb = false>
 __device__ __forceinline__ void leafparent_body(Ctx x, Blocks blk) {
   static_assert(Lanes == 2 || Lanes == 4 || Lanes == 8, "2, 4 or 8 lanes per item");
   constexpr uint32_t kPer = 8 / Lanes; // leaves per lane
@@ -342,11 +335,8 @@ __device__ __forceinline__ void leafparent_body(Ctx x, Blocks blk) {
 #pragma unroll
     for (uint32_t j = 0; j < kPer; ++j) result[j] = old_child[j] = kEmptyRef;
     Item it{};
-    uint32_t next_old = kEmptyRef; // Prefetch: the old ref of the group's next item
     if (have) {
       it = x.a.items[base + wi];
-      if (Prefetch && q == 0 && g + stride < total)
-        next_old = x.a.items[base + static_cast<uint32_t>((g + stride) / Lanes)].old;
       const Cell cell = unpack_cell(it.cell);
       // Independent loads side by side: the first chunk's pair index and the
       // old node, then its primitive and the old leaves (read speculatively:
@@ -373,7 +363,6 @@ __device__ __forceinline__ void leafparent_body(Ctx x, Blocks blk) {
         mask[j] = 0;
         loaded[j] = touched[j] = false;
       }
-      if (Prefetch && next_old > kFullRef) prefetch_l2(x.t.pool[l] + (next_old - 2u));
       __syncwarp(gmask); // the group's previous item no longer reads s_pr
       s_pr[grp][q] = first;
       __syncwarp(gmask);
@@ -430,9 +419,149 @@ __device__ __forceinline__ void leafparent_body(Ctx x, Blocks blk) {
   }
 }
 
-template <bool Terrain, int MinBlocks, uint32_t Lanes, bool Prefetch = false>
+// (eight lanes per item, registers for four blocks: the generator's leaf
+// masks need them)
+__global__ void __launch_bounds__(kBlock, 4) leafparent_terrain_kernel(Ctx x) {
+  leafparent_body<true, 8>(x, launch_blocks());
+}
+
+// The same level for edits, a warp taking 32 items at a time: each lane owns
+// an item for what is done once per item (its record, its first primitive,
+// the old node, the classification of its 8 leaves, the hash-consing of the
+// new node), and the leaves that some primitive touches are listed and dealt
+// out to the lanes, so that the expensive part, a leaf's mask and its probe,
+// runs with full warps.  Nearly every item of a batch has one primitive
+// (24.82 M primitives for 24.78 M items at 16,384 spheres in 16384^3), whose
+// classification tells which leaves those are; the leaves of an item with
+// more are all listed and walk its list.
+//
+// What bounds it: dependent random reads (item, old node, old leaf, leaf
+// probe, node probe, item compare), so 32 items of a warp wait together where
+// four lanes per item kept 8 in flight, and the integer and FMA pipes, whose
+// work per item is a third of what it was (a touched leaf in four lanes'
+// stride idled the others, and hashing ran on one lane in four).  On B200,
+// 24.8 M items: 4.58 ms with four lanes per item, 2.65 ms so (2.79 built for
+// four resident blocks, 2.61 for six).
+// MinBlocks: the knob "edit.leafparent_blocks".  Prefetch (the knob
+// "edit.leafparent_prefetch"): the old node of the lane's next item is
+// prefetched into L2.
+struct WarpLeaves {
+  uint32_t ref[8][kWarp];   // [child][item]: old child ref, then the new one
+  vx_primitive prim[kWarp]; // the items' first primitives
+  uint8_t task[8 * kWarp];  // item | child << 5
+  uint8_t changed[kWarp];   // the item has a child with a new ref
+};
+
+template <int MinBlocks, bool Prefetch>
 __global__ void __launch_bounds__(kBlock, MinBlocks) leafparent_kernel(Ctx x) {
-  leafparent_body<Terrain, Lanes, false, Prefetch>(x, launch_blocks());
+  __shared__ WarpLeaves s_warp[kBlock / kWarp];
+  Header *h = x.t.hdr;
+  const uint32_t l = x.t.depth - 1;
+  const uint32_t W = h->item_count[l]; // loaded beside the status
+  const uint32_t base = h->item_off[l];
+  if (edit_failed(h)) return;
+  const uint32_t *pairs = x.a.pairs[l & 1u];
+  const uint32_t world_exp = x.t.depth + 2;
+  const uint32_t lane = lane_id();
+  WarpLeaves &s = s_warp[threadIdx.x / kWarp];
+  const uint32_t stride = gridDim.x * kBlock;
+  for (uint64_t w0 = blockIdx.x * uint64_t(kBlock) + threadIdx.x - lane; w0 < W; w0 += stride) {
+    const uint32_t wi = static_cast<uint32_t>(w0) + lane;
+    const bool have = w0 + lane < W;
+    Item it{};
+    uint32_t touched = 0;
+    if (have) {
+      it = x.a.items[base + wi];
+      uint32_t next_old = kEmptyRef;
+      if (Prefetch && w0 + lane + stride < W) next_old = x.a.items[base + wi + stride].old;
+      const uint32_t pidx = it.pcount != 0 ? pairs[it.pstart] : 0u;
+      // old children (the header and its refs lie in one or two sectors)
+      if (it.old <= kFullRef) {
+#pragma unroll
+        for (uint32_t c = 0; c < 8; ++c) s.ref[c][lane] = it.old;
+      } else {
+        const uint32_t *node = x.t.pool[l] + (it.old - 2u);
+        const uint32_t header = node[0];
+#pragma unroll
+        for (uint32_t c = 0; c < 8; ++c) {
+          const uint32_t bit = 1u << c;
+          uint32_t r = (header >> (8u + c)) & 1u; // kFullRef or kEmptyRef
+          if (header & bit) r = node[1u + __popc(header & (bit - 1u))];
+          s.ref[c][lane] = r;
+        }
+      }
+      if (Prefetch && next_old > kFullRef) prefetch_l2(x.t.pool[l] + (next_old - 2u));
+      if (it.pcount == 1) {
+        const vx_primitive pr = x.prims[pidx];
+        s.prim[lane] = pr;
+        const Cell cell = unpack_cell(it.cell);
+        if (vx_prim_shape(&pr) == VX_SHAPE_SPHERE && pr.r[0] < kFastRadius) {
+          uint32_t covered;
+          sphere_classify_leaves(pr, cell.x * 8u, cell.y * 8u, cell.z * 8u, touched, covered);
+        } else {
+          for (uint32_t c = 0; c < 8; ++c)
+            if (classify<false>(pr, world_exp, int64_t(2 * cell.x + (c & 1u)) * 4,
+                                int64_t(2 * cell.y + ((c >> 1) & 1u)) * 4,
+                                int64_t(2 * cell.z + (c >> 2)) * 4, 4) != VX_CELL_EMPTY)
+              touched |= 1u << c;
+        }
+      } else if (it.pcount > 1) {
+        s.prim[lane] = x.prims[pidx];
+        touched = 0xffu;
+      }
+    }
+    s.changed[lane] = 0;
+    // The touched leaves of all items, listed item by item.
+    const uint32_t mine = __popc(touched);
+    const uint32_t inc = warp_inclusive_sum(mine);
+    const uint32_t tasks = __shfl_sync(kFullMask, inc, kWarp - 1);
+    uint32_t at = inc - mine;
+    for (uint32_t m = touched; m != 0u; m &= m - 1u)
+      s.task[at++] = static_cast<uint8_t>(lane | ((__ffs(m) - 1u) << 5));
+    __syncwarp();
+    for (uint32_t t0 = 0; t0 < tasks; t0 += kWarp) {
+      const bool busy = t0 + lane < tasks;
+      const uint32_t task = busy ? s.task[t0 + lane] : 0u;
+      const uint32_t src = task & 31u, c = task >> 5;
+      const uint64_t cell_bits = __shfl_sync(kFullMask, it.cell, src);
+      const uint32_t pstart = __shfl_sync(kFullMask, it.pstart, src);
+      const uint32_t pcount = __shfl_sync(kFullMask, it.pcount, src);
+      if (!busy) continue;
+      const uint32_t old_ref = s.ref[c][src];
+      const uint64_t old_mask = read_leaf(x.t, old_ref);
+      const Cell cell = unpack_cell(cell_bits);
+      const int64_t ox = int64_t(2 * cell.x + (c & 1u)) * 4;
+      const int64_t oy = int64_t(2 * cell.y + ((c >> 1) & 1u)) * 4;
+      const int64_t oz = int64_t(2 * cell.z + (c >> 2)) * 4;
+      uint64_t mask = old_mask;
+      for (uint32_t k = 0; k < pcount; ++k) {
+        const vx_primitive pr = k == 0 ? s.prim[src] : x.prims[pairs[pstart + k]];
+        const uint32_t cls = classify<false>(pr, world_exp, ox, oy, oz, 4);
+        if (cls == VX_CELL_EMPTY) continue;
+        const uint64_t m = cls == VX_CELL_FULL ? ~0ull : leaf_mask<false>(pr, world_exp, ox, oy, oz);
+        mask = vx_prim_op(&pr) == VX_OP_ADD ? (mask | m) : (mask & ~m);
+      }
+      // An unchanged mask keeps its canonical ref: no probe of the leaf set.
+      if (mask != old_mask) {
+        s.ref[c][src] = canon_leaf(x.t, mask);
+        s.changed[src] = 1;
+      }
+    }
+    __syncwarp();
+    // A node whose 8 children all kept their refs is the old node itself
+    // (refs are canonical), so its hash-consing is skipped.
+    if (have) {
+      uint32_t result = it.old;
+      if (s.changed[lane]) {
+        uint32_t child[8];
+#pragma unroll
+        for (uint32_t c = 0; c < 8; ++c) child[c] = s.ref[c][lane];
+        result = canon_node(x.t, l, child);
+      }
+      x.a.items[base + wi].result = result;
+    }
+    __syncwarp(); // the next items overwrite the warp's buffers
+  }
 }
 
 // The rebuilt ref of one item at inner level l from its children's results.
@@ -892,35 +1021,12 @@ vx_status run_pipeline(vx_dag *d, const vx_primitive *prims,
   {
     prof::Scope sc("dag_leafparent", s);
     const int64_t lb = tune::get(tune::kEditLeafparentBlocks);
-    const int64_t lanes = tune::get(tune::kEditLeafparentLanes);
-    const bool four = lanes == 4;
     const bool prefetch = tune::get(tune::kEditLeafparentPrefetch) != 0;
-    if (terrain)
-      leafparent_kernel<true, 4, 8><<<grid, kBlock, 0, s>>>(x);
-    else if (four && prefetch && lb == 6)
-      leafparent_kernel<false, 6, 4, true><<<grid, kBlock, 0, s>>>(x);
-    else if (four && prefetch && lb == 5)
-      leafparent_kernel<false, 5, 4, true><<<grid, kBlock, 0, s>>>(x);
-    else if (four && prefetch)
-      leafparent_kernel<false, 4, 4, true><<<grid, kBlock, 0, s>>>(x);
-    else if (lanes == 2 && lb == 6)
-      leafparent_kernel<false, 6, 2><<<grid, kBlock, 0, s>>>(x);
-    else if (lanes == 2 && lb == 5)
-      leafparent_kernel<false, 5, 2><<<grid, kBlock, 0, s>>>(x);
-    else if (lanes == 2)
-      leafparent_kernel<false, 4, 2><<<grid, kBlock, 0, s>>>(x);
-    else if (four && lb == 6)
-      leafparent_kernel<false, 6, 4><<<grid, kBlock, 0, s>>>(x);
-    else if (four && lb == 5)
-      leafparent_kernel<false, 5, 4><<<grid, kBlock, 0, s>>>(x);
-    else if (four)
-      leafparent_kernel<false, 4, 4><<<grid, kBlock, 0, s>>>(x);
-    else if (lb == 6)
-      leafparent_kernel<false, 6, 8><<<grid, kBlock, 0, s>>>(x);
-    else if (lb == 5)
-      leafparent_kernel<false, 5, 8><<<grid, kBlock, 0, s>>>(x);
-    else
-      leafparent_kernel<false, 4, 8><<<grid, kBlock, 0, s>>>(x);
+    auto launch = [&](auto kernel) { kernel<<<grid, kBlock, 0, s>>>(x); };
+    if (terrain) launch(leafparent_terrain_kernel);
+    else if (lb == 6) launch(prefetch ? leafparent_kernel<6, true> : leafparent_kernel<6, false>);
+    else if (lb == 5) launch(prefetch ? leafparent_kernel<5, true> : leafparent_kernel<5, false>);
+    else launch(prefetch ? leafparent_kernel<4, true> : leafparent_kernel<4, false>);
   }
   VX_TRY_CUDA(cudaGetLastError());
   for (uint32_t r = depth - 1; r > 0; --r) {

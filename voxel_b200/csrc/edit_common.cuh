@@ -113,9 +113,8 @@ __device__ __forceinline__ uint64_t sphere_leaf_mask32(const vx_primitive &p, in
 // which each single-precision operation (contracted or not) keeps exact.  A
 // voxel is inside when sx <= r^2 - sy - sz, i.e. when sx - (r^2 + 1 - sy -
 // sz) is negative; an exact zero is +0, so the sign bit is the voxel's bit.
-// The sign bits of a row's four voxels are gathered by byte permutes and one
-// multiply (bits 7, 15, 23, 31 land in bits 28-31 with no carries into
-// them), which moves most of the work off the integer pipe.
+// The sign bits are shifted into the mask one funnel shift per voxel, the
+// highest voxel first: a subtraction and a shift per voxel.
 constexpr uint32_t kFloatMaskRadius = 1024;
 
 __device__ __forceinline__ uint64_t sphere_leaf_mask_f32(const vx_primitive &p, int64_t ox,
@@ -134,20 +133,54 @@ __device__ __forceinline__ uint64_t sphere_leaf_mask_f32(const vx_primitive &p, 
   const float r2p1 = r * r + 1.0f;
   uint32_t half[2] = {0u, 0u};
 #pragma unroll
-  for (int z = 0; z < 4; ++z) {
+  for (int z = 3; z >= 0; --z) {
     const float c = fz + static_cast<float>(z);
     const float tz = r2p1 - c * c;
 #pragma unroll
-    for (int y = 0; y < 4; ++y) {
+    for (int y = 3; y >= 0; --y) {
       const float t = tz - sy[y];
-      const uint32_t d01 = __byte_perm(__float_as_uint(sx[0] - t), __float_as_uint(sx[1] - t), 0x0073);
-      const uint32_t d23 = __byte_perm(__float_as_uint(sx[2] - t), __float_as_uint(sx[3] - t), 0x0073);
-      const uint32_t w = __byte_perm(d01, d23, 0x5410); // byte x = the top byte of voxel x's value
-      const uint32_t row = ((w & 0x80808080u) * 0x00204081u) >> 28;
-      half[z >> 1] |= row << (4 * y + 16 * (z & 1));
+#pragma unroll
+      for (int i = 3; i >= 0; --i)
+        half[z >> 1] = __funnelshift_l(__float_as_uint(sx[i] - t), half[z >> 1], 1);
     }
   }
   return (static_cast<uint64_t>(half[1]) << 32) | half[0];
+}
+
+// Leaves of the 8^3 cell at o (a leaf parent's cell) that a sphere of radius
+// below kFastRadius touches and covers, one bit per child: the nearest and
+// farthest squared distances per axis are found once for each half of the
+// cell and summed per child (sphere_classify32 leaf by leaf costs four times
+// the instructions).  Distances are clamped to r + 1, which keeps every
+// square and sum below 2^31 and every outcome.
+__device__ __forceinline__ void sphere_classify_leaves(const vx_primitive &p, uint32_t ox,
+                                                       uint32_t oy, uint32_t oz, uint32_t &touched,
+                                                       uint32_t &covered) {
+  const int32_t r = static_cast<int32_t>(p.r[0]);
+  const int32_t lo[3] = {static_cast<int32_t>(ox), static_cast<int32_t>(oy),
+                         static_cast<int32_t>(oz)};
+  int32_t near2[3][2], far2[3][2];
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    const int32_t c = max(-(1 << 16), min(1 << 18, p.c[a]));
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int32_t a0 = lo[a] + 4 * h, a1 = a0 + 3;
+      const int32_t d = min(max(max(a0 - c, c - a1), 0), r + 1);
+      const int32_t f = min(max(c - a0, a1 - c), r + 1); // the farther end
+      near2[a][h] = d * d;
+      far2[a][h] = f * f;
+    }
+  }
+  const int32_t r2 = r * r;
+  touched = covered = 0;
+#pragma unroll
+  for (uint32_t c = 0; c < 8; ++c) {
+    const int32_t n = near2[0][c & 1u] + near2[1][(c >> 1) & 1u] + near2[2][c >> 2];
+    const int32_t f = far2[0][c & 1u] + far2[1][(c >> 1) & 1u] + far2[2][c >> 2];
+    if (n <= r2) touched |= 1u << c;
+    if (f <= r2) covered |= 1u << c;
+  }
 }
 
 // Classify primitive p against the voxel cube [o, o + n)^3.  Kernels that
