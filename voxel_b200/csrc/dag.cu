@@ -446,11 +446,45 @@ __global__ void __launch_bounds__(kBlock, 4) leafparent_terrain_kernel(Ctx x) {
 // "edit.leafparent_prefetch"): the old node of the lane's next item is
 // prefetched into L2.
 struct WarpLeaves {
-  uint32_t ref[8][kWarp];   // [child][item]: old child ref, then the new one
-  vx_primitive prim[kWarp]; // the items' first primitives
-  uint8_t task[8 * kWarp];  // item | child << 5
-  uint8_t changed[kWarp];   // the item has a child with a new ref
+  uint32_t ref[8][kWarp];  // [child][item]: old child ref, then the new one
+  float4 ball[kWarp];      // of an item with one sphere: the cell's first voxel
+                           // relative to its centre, and r^2 + 1
+  uint8_t task[8 * kWarp]; // item | child << 5
+  uint8_t changed[kWarp];  // the item has a child with a new ref
 };
+
+// The two less usual branches are functions of their own, so that their
+// registers do not weigh on the loop: leaves of `cell` that a primitive other
+// than a sphere touches, and the mask of leaf c of `cell` after a whole list.
+__device__ __noinline__ uint32_t touched_leaves(const vx_primitive *p, uint64_t cell,
+                                                uint32_t world_exp) {
+  const Cell k = unpack_cell(cell);
+  const vx_primitive pr = *p;
+  uint32_t touched = 0;
+  for (uint32_t c = 0; c < 8; ++c)
+    if (classify<false>(pr, world_exp, int64_t(2 * k.x + (c & 1u)) * 4,
+                        int64_t(2 * k.y + ((c >> 1) & 1u)) * 4, int64_t(2 * k.z + (c >> 2)) * 4,
+                        4) != VX_CELL_EMPTY)
+      touched |= 1u << c;
+  return touched;
+}
+
+__device__ __noinline__ uint64_t list_leaf_mask(const vx_primitive *prims, const uint32_t *list,
+                                                uint32_t count, uint64_t cell, uint32_t c,
+                                                uint32_t world_exp, uint64_t mask) {
+  const Cell k = unpack_cell(cell);
+  const int64_t ox = int64_t(2 * k.x + (c & 1u)) * 4;
+  const int64_t oy = int64_t(2 * k.y + ((c >> 1) & 1u)) * 4;
+  const int64_t oz = int64_t(2 * k.z + (c >> 2)) * 4;
+  for (uint32_t i = 0; i < count; ++i) {
+    const vx_primitive pr = prims[list[i]];
+    const uint32_t cls = classify<false>(pr, world_exp, ox, oy, oz, 4);
+    if (cls == VX_CELL_EMPTY) continue;
+    const uint64_t m = cls == VX_CELL_FULL ? ~0ull : leaf_mask<false>(pr, world_exp, ox, oy, oz);
+    mask = vx_prim_op(&pr) == VX_OP_ADD ? (mask | m) : (mask & ~m);
+  }
+  return mask;
+}
 
 template <int MinBlocks, bool Prefetch>
 __global__ void __launch_bounds__(kBlock, MinBlocks) leafparent_kernel(Ctx x) {
@@ -470,6 +504,7 @@ __global__ void __launch_bounds__(kBlock, MinBlocks) leafparent_kernel(Ctx x) {
     const bool have = w0 + lane < W;
     Item it{};
     uint32_t touched = 0;
+    uint32_t info = 0; // covered children | one sphere << 8 | add << 9
     if (have) {
       it = x.a.items[base + wi];
       uint32_t next_old = kEmptyRef;
@@ -493,20 +528,20 @@ __global__ void __launch_bounds__(kBlock, MinBlocks) leafparent_kernel(Ctx x) {
       if (Prefetch && next_old > kFullRef) prefetch_l2(x.t.pool[l] + (next_old - 2u));
       if (it.pcount == 1) {
         const vx_primitive pr = x.prims[pidx];
-        s.prim[lane] = pr;
         const Cell cell = unpack_cell(it.cell);
-        if (vx_prim_shape(&pr) == VX_SHAPE_SPHERE && pr.r[0] < kFastRadius) {
-          uint32_t covered;
-          sphere_classify_leaves(pr, cell.x * 8u, cell.y * 8u, cell.z * 8u, touched, covered);
+        if (vx_prim_shape(&pr) == VX_SHAPE_SPHERE && pr.r[0] <= kFloatMaskRadius) {
+          sphere_classify_leaves(pr, cell.x * 8u, cell.y * 8u, cell.z * 8u, touched, info);
+          info |= vx_prim_op(&pr) == VX_OP_ADD ? 0x300u : 0x100u;
+          const float r = static_cast<float>(pr.r[0]);
+          s.ball[lane] =
+              make_float4(static_cast<float>(static_cast<int32_t>(cell.x * 8u) - pr.c[0]),
+                          static_cast<float>(static_cast<int32_t>(cell.y * 8u) - pr.c[1]),
+                          static_cast<float>(static_cast<int32_t>(cell.z * 8u) - pr.c[2]),
+                          r * r + 1.0f);
         } else {
-          for (uint32_t c = 0; c < 8; ++c)
-            if (classify<false>(pr, world_exp, int64_t(2 * cell.x + (c & 1u)) * 4,
-                                int64_t(2 * cell.y + ((c >> 1) & 1u)) * 4,
-                                int64_t(2 * cell.z + (c >> 2)) * 4, 4) != VX_CELL_EMPTY)
-              touched |= 1u << c;
+          touched = touched_leaves(x.prims + pidx, it.cell, world_exp);
         }
       } else if (it.pcount > 1) {
-        s.prim[lane] = x.prims[pidx];
         touched = 0xffu;
       }
     }
@@ -523,26 +558,31 @@ __global__ void __launch_bounds__(kBlock, MinBlocks) leafparent_kernel(Ctx x) {
       const bool busy = t0 + lane < tasks;
       const uint32_t task = busy ? s.task[t0 + lane] : 0u;
       const uint32_t src = task & 31u, c = task >> 5;
-      const uint64_t cell_bits = __shfl_sync(kFullMask, it.cell, src);
-      const uint32_t pstart = __shfl_sync(kFullMask, it.pstart, src);
-      const uint32_t pcount = __shfl_sync(kFullMask, it.pcount, src);
-      if (!busy) continue;
-      const uint32_t old_ref = s.ref[c][src];
-      const uint64_t old_mask = read_leaf(x.t, old_ref);
-      const Cell cell = unpack_cell(cell_bits);
-      const int64_t ox = int64_t(2 * cell.x + (c & 1u)) * 4;
-      const int64_t oy = int64_t(2 * cell.y + ((c >> 1) & 1u)) * 4;
-      const int64_t oz = int64_t(2 * cell.z + (c >> 2)) * 4;
-      uint64_t mask = old_mask;
-      for (uint32_t k = 0; k < pcount; ++k) {
-        const vx_primitive pr = k == 0 ? s.prim[src] : x.prims[pairs[pstart + k]];
-        const uint32_t cls = classify<false>(pr, world_exp, ox, oy, oz, 4);
-        if (cls == VX_CELL_EMPTY) continue;
-        const uint64_t m = cls == VX_CELL_FULL ? ~0ull : leaf_mask<false>(pr, world_exp, ox, oy, oz);
-        mask = vx_prim_op(&pr) == VX_OP_ADD ? (mask | m) : (mask & ~m);
+      const uint32_t src_info = __shfl_sync(kFullMask, info, src);
+      const bool one_sphere = (src_info & 0x100u) != 0;
+      uint32_t old_ref = kEmptyRef;
+      uint64_t old_mask = 0, mask = 0;
+      if (busy) {
+        old_ref = s.ref[c][src];
+        mask = old_mask = read_leaf(x.t, old_ref);
+      }
+      if (busy && one_sphere) {
+        const float4 b = s.ball[src];
+        uint64_t m = ~0ull;
+        if (((src_info >> c) & 1u) == 0u)
+          m = sphere_mask_rows(b.x + ((c & 1u) ? 4.0f : 0.0f), b.y + ((c & 2u) ? 4.0f : 0.0f),
+                               b.z + ((c & 4u) ? 4.0f : 0.0f), b.w);
+        mask = (src_info & 0x200u) ? (mask | m) : (mask & ~m);
+      }
+      if (__any_sync(kFullMask, busy && !one_sphere)) { // other shapes, longer lists
+        const uint64_t cell_bits = __shfl_sync(kFullMask, it.cell, src);
+        const uint32_t pstart = __shfl_sync(kFullMask, it.pstart, src);
+        const uint32_t pcount = __shfl_sync(kFullMask, it.pcount, src);
+        if (busy && !one_sphere)
+          mask = list_leaf_mask(x.prims, pairs + pstart, pcount, cell_bits, c, world_exp, mask);
       }
       // An unchanged mask keeps its canonical ref: no probe of the leaf set.
-      if (mask != old_mask) {
+      if (busy && mask != old_mask) {
         s.ref[c][src] = canon_leaf(x.t, mask);
         s.changed[src] = 1;
       }

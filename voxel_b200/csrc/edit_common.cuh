@@ -117,12 +117,8 @@ __device__ __forceinline__ uint64_t sphere_leaf_mask32(const vx_primitive &p, in
 // highest voxel first: a subtraction and a shift per voxel.
 constexpr uint32_t kFloatMaskRadius = 1024;
 
-__device__ __forceinline__ uint64_t sphere_leaf_mask_f32(const vx_primitive &p, int64_t ox,
-                                                        int64_t oy, int64_t oz) {
-  const float r = static_cast<float>(p.r[0]);
-  const float fx = static_cast<float>(static_cast<int32_t>(ox - p.c[0]));
-  const float fy = static_cast<float>(static_cast<int32_t>(oy - p.c[1]));
-  const float fz = static_cast<float>(static_cast<int32_t>(oz - p.c[2]));
+// (fx, fy, fz): the leaf's first voxel relative to the centre; r2p1 = r^2 + 1.
+__device__ __forceinline__ uint64_t sphere_mask_rows(float fx, float fy, float fz, float r2p1) {
   float sx[4], sy[4];
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
@@ -130,7 +126,6 @@ __device__ __forceinline__ uint64_t sphere_leaf_mask_f32(const vx_primitive &p, 
     sx[i] = a * a;
     sy[i] = b * b;
   }
-  const float r2p1 = r * r + 1.0f;
   uint32_t half[2] = {0u, 0u};
 #pragma unroll
   for (int z = 3; z >= 0; --z) {
@@ -145,6 +140,14 @@ __device__ __forceinline__ uint64_t sphere_leaf_mask_f32(const vx_primitive &p, 
     }
   }
   return (static_cast<uint64_t>(half[1]) << 32) | half[0];
+}
+
+__device__ __forceinline__ uint64_t sphere_leaf_mask_f32(const vx_primitive &p, int64_t ox,
+                                                        int64_t oy, int64_t oz) {
+  const float r = static_cast<float>(p.r[0]);
+  return sphere_mask_rows(static_cast<float>(static_cast<int32_t>(ox - p.c[0])),
+                          static_cast<float>(static_cast<int32_t>(oy - p.c[1])),
+                          static_cast<float>(static_cast<int32_t>(oz - p.c[2])), r * r + 1.0f);
 }
 
 // Leaves of the 8^3 cell at o (a leaf parent's cell) that a sphere of radius
