@@ -278,6 +278,21 @@ struct DagTree {
   __device__ uint32_t child(uint32_t l, uint32_t ref, uint32_t c) const {
     return child_ref(t, l, ref, c);
   }
+  __device__ __forceinline__ void children(uint32_t l, uint32_t ref, uint32_t (&out)[8]) const {
+    if (ref <= kFullRef) {
+#pragma unroll
+      for (uint32_t c = 0; c < 8; ++c) out[c] = ref;
+      return;
+    }
+    const uint32_t *node = t.pool[l] + (ref - 2u);
+    const uint32_t header = node[0];
+#pragma unroll
+    for (uint32_t c = 0; c < 8; ++c) {
+      const uint32_t bit = 1u << c;
+      out[c] = (header >> (8u + c)) & 1u; // kFullRef or kEmptyRef
+      if (header & bit) out[c] = node[1u + __popc(header & (bit - 1u))];
+    }
+  }
   // Superseded subtrees stay in the tables until vx_dag_compact.
   __device__ void replaced(uint32_t, uint32_t, uint32_t) const {}
   template <bool Terrain>
@@ -453,22 +468,8 @@ struct WarpLeaves {
   uint8_t changed[kWarp];  // the item has a child with a new ref
 };
 
-// The two less usual branches are functions of their own, so that their
-// registers do not weigh on the loop: leaves of `cell` that a primitive other
-// than a sphere touches, and the mask of leaf c of `cell` after a whole list.
-__device__ __noinline__ uint32_t touched_leaves(const vx_primitive *p, uint64_t cell,
-                                                uint32_t world_exp) {
-  const Cell k = unpack_cell(cell);
-  const vx_primitive pr = *p;
-  uint32_t touched = 0;
-  for (uint32_t c = 0; c < 8; ++c)
-    if (classify<false>(pr, world_exp, int64_t(2 * k.x + (c & 1u)) * 4,
-                        int64_t(2 * k.y + ((c >> 1) & 1u)) * 4, int64_t(2 * k.z + (c >> 2)) * 4,
-                        4) != VX_CELL_EMPTY)
-      touched |= 1u << c;
-  return touched;
-}
-
+// The mask of leaf c of `cell` after a whole list; a function of its own, so
+// that its registers do not weigh on the loop.
 __device__ __noinline__ uint64_t list_leaf_mask(const vx_primitive *prims, const uint32_t *list,
                                                 uint32_t count, uint64_t cell, uint32_t c,
                                                 uint32_t world_exp, uint64_t mask) {
@@ -498,6 +499,7 @@ __global__ void __launch_bounds__(kBlock, MinBlocks) leafparent_kernel(Ctx x) {
   const uint32_t world_exp = x.t.depth + 2;
   const uint32_t lane = lane_id();
   WarpLeaves &s = s_warp[threadIdx.x / kWarp];
+  const DagTree tree{x.t};
   const uint32_t stride = gridDim.x * kBlock;
   for (uint64_t w0 = blockIdx.x * uint64_t(kBlock) + threadIdx.x - lane; w0 < W; w0 += stride) {
     const uint32_t wi = static_cast<uint32_t>(w0) + lane;
@@ -510,27 +512,16 @@ __global__ void __launch_bounds__(kBlock, MinBlocks) leafparent_kernel(Ctx x) {
       uint32_t next_old = kEmptyRef;
       if (Prefetch && w0 + lane + stride < W) next_old = x.a.items[base + wi + stride].old;
       const uint32_t pidx = it.pcount != 0 ? pairs[it.pstart] : 0u;
-      // old children (the header and its refs lie in one or two sectors)
-      if (it.old <= kFullRef) {
+      uint32_t old_child[8];
+      tree.children(l, it.old, old_child);
 #pragma unroll
-        for (uint32_t c = 0; c < 8; ++c) s.ref[c][lane] = it.old;
-      } else {
-        const uint32_t *node = x.t.pool[l] + (it.old - 2u);
-        const uint32_t header = node[0];
-#pragma unroll
-        for (uint32_t c = 0; c < 8; ++c) {
-          const uint32_t bit = 1u << c;
-          uint32_t r = (header >> (8u + c)) & 1u; // kFullRef or kEmptyRef
-          if (header & bit) r = node[1u + __popc(header & (bit - 1u))];
-          s.ref[c][lane] = r;
-        }
-      }
+      for (uint32_t c = 0; c < 8; ++c) s.ref[c][lane] = old_child[c];
       if (Prefetch && next_old > kFullRef) prefetch_l2(x.t.pool[l] + (next_old - 2u));
       if (it.pcount == 1) {
         const vx_primitive pr = x.prims[pidx];
         const Cell cell = unpack_cell(it.cell);
         if (vx_prim_shape(&pr) == VX_SHAPE_SPHERE && pr.r[0] <= kFloatMaskRadius) {
-          sphere_classify_leaves(pr, cell.x * 8u, cell.y * 8u, cell.z * 8u, touched, info);
+          sphere_classify_children(pr, cell.x * 8u, cell.y * 8u, cell.z * 8u, 4u, touched, info);
           info |= vx_prim_op(&pr) == VX_OP_ADD ? 0x300u : 0x100u;
           const float r = static_cast<float>(pr.r[0]);
           s.ball[lane] =
@@ -539,7 +530,7 @@ __global__ void __launch_bounds__(kBlock, MinBlocks) leafparent_kernel(Ctx x) {
                           static_cast<float>(static_cast<int32_t>(cell.z * 8u) - pr.c[2]),
                           r * r + 1.0f);
         } else {
-          touched = touched_leaves(x.prims + pidx, it.cell, world_exp);
+          touched = other_children(x.prims + pidx, it.cell, 4u) & 0xffu;
         }
       } else if (it.pcount > 1) {
         touched = 0xffu;
@@ -1038,7 +1029,8 @@ vx_status run_pipeline(vx_dag *d, const vx_primitive *prims,
       else if (sorted_keys != nullptr)
         expand_sorted_kernel<DagTree><<<lgrid, kBlock, 0, s>>>(e, tree, l);
       else
-        expand_kernel<DagTree, false><<<lgrid, kBlock, 0, s>>>(e, tree, l);
+        expand_warp_kernel<DagTree>
+            <<<level_grid(grid, l, kBlock), kBlock, 0, s>>>(e, tree, l);
     }
     VX_TRY_CUDA(cudaGetLastError());
     if (sorted_keys != nullptr) continue;

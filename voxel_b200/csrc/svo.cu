@@ -92,6 +92,18 @@ struct SvoTree {
     if (old & kChild) return t.nodes[static_cast<size_t>(old & kIndex) * 8u + c];
     return old; // a uniform region's children hold the same value
   }
+  __device__ __forceinline__ void children(uint32_t, uint32_t old, uint32_t (&out)[8]) const {
+    if (!(old & kChild)) {
+#pragma unroll
+      for (uint32_t c = 0; c < 8; ++c) out[c] = old;
+      return;
+    }
+    const uint4 *src =
+        reinterpret_cast<const uint4 *>(t.nodes + static_cast<size_t>(old & kIndex) * 8u);
+    const uint4 a = src[0], b = src[1];
+    out[0] = a.x; out[1] = a.y; out[2] = a.z; out[3] = a.w;
+    out[4] = b.x; out[5] = b.y; out[6] = b.z; out[7] = b.w;
+  }
   // A materialised child overwritten by a covering primitive leaves its
   // subtree unreachable: flag it for a later collection.
   __device__ void replaced(uint32_t l, uint32_t old, uint32_t c) const {
@@ -809,7 +821,9 @@ vx_status run_pipeline(vx_svo *v, const vx_primitive *prims, const uint32_t *d_c
       prof::Scope sc("svo_expand", s);
       if (terrain) expand_kernel<SvoTree, true><<<lgrid, kBlock, 0, s>>>(e, pol, l);
       else if (sorted_keys) expand_sorted_kernel<SvoTree><<<lgrid, kBlock, 0, s>>>(e, pol, l);
-      else expand_kernel<SvoTree, false><<<lgrid, kBlock, 0, s>>>(e, pol, l);
+      else
+        expand_warp_kernel<SvoTree>
+            <<<level_grid(grid, l, kBlock), kBlock, 0, s>>>(e, pol, l);
     }
     VX_TRY_CUDA(cudaGetLastError());
     if (sorted_keys != nullptr) continue;
