@@ -270,6 +270,7 @@ struct Ctx {
   const vx_primitive *prims;
   const uint32_t *d_prim_count; // device count (NULL: use host_prim_count)
   uint32_t host_prim_count;
+  const uint64_t *sorted_keys; // EditCtx::sorted_keys
 };
 
 struct DagTree {
@@ -468,25 +469,6 @@ struct WarpLeaves {
   uint8_t changed[kWarp];  // the item has a child with a new ref
 };
 
-// The mask of leaf c of `cell` after a whole list; a function of its own, so
-// that its registers do not weigh on the loop.
-__device__ __noinline__ uint64_t list_leaf_mask(const vx_primitive *prims, const uint32_t *list,
-                                                uint32_t count, uint64_t cell, uint32_t c,
-                                                uint32_t world_exp, uint64_t mask) {
-  const Cell k = unpack_cell(cell);
-  const int64_t ox = int64_t(2 * k.x + (c & 1u)) * 4;
-  const int64_t oy = int64_t(2 * k.y + ((c >> 1) & 1u)) * 4;
-  const int64_t oz = int64_t(2 * k.z + (c >> 2)) * 4;
-  for (uint32_t i = 0; i < count; ++i) {
-    const vx_primitive pr = prims[list[i]];
-    const uint32_t cls = classify<false>(pr, world_exp, ox, oy, oz, 4);
-    if (cls == VX_CELL_EMPTY) continue;
-    const uint64_t m = cls == VX_CELL_FULL ? ~0ull : leaf_mask<false>(pr, world_exp, ox, oy, oz);
-    mask = vx_prim_op(&pr) == VX_OP_ADD ? (mask | m) : (mask & ~m);
-  }
-  return mask;
-}
-
 template <int MinBlocks, bool Prefetch>
 __global__ void __launch_bounds__(kBlock, MinBlocks) leafparent_kernel(Ctx x) {
   __shared__ WarpLeaves s_warp[kBlock / kWarp];
@@ -496,7 +478,6 @@ __global__ void __launch_bounds__(kBlock, MinBlocks) leafparent_kernel(Ctx x) {
   const uint32_t base = h->item_off[l];
   if (edit_failed(h)) return;
   const uint32_t *pairs = x.a.pairs[l & 1u];
-  const uint32_t world_exp = x.t.depth + 2;
   const uint32_t lane = lane_id();
   WarpLeaves &s = s_warp[threadIdx.x / kWarp];
   const DagTree tree{x.t};
@@ -506,7 +487,7 @@ __global__ void __launch_bounds__(kBlock, MinBlocks) leafparent_kernel(Ctx x) {
     const bool have = w0 + lane < W;
     Item it{};
     uint32_t touched = 0;
-    uint32_t info = 0; // covered children | one sphere << 8 | add << 9
+    uint32_t info = 0; // covered children | one sphere << 8 | add << 9 | sorted leaf masks << 10
     if (have) {
       it = x.a.items[base + wi];
       uint32_t next_old = kEmptyRef;
@@ -517,7 +498,11 @@ __global__ void __launch_bounds__(kBlock, MinBlocks) leafparent_kernel(Ctx x) {
 #pragma unroll
       for (uint32_t c = 0; c < 8; ++c) s.ref[c][lane] = old_child[c];
       if (Prefetch && next_old > kFullRef) prefetch_l2(x.t.pool[l] + (next_old - 2u));
-      if (it.pcount == 1) {
+      if (x.sorted_keys != nullptr) { // a leaf mask per touched leaf, in child order
+        for (uint32_t k = 0; k < it.pcount; ++k)
+          touched |= 1u << (static_cast<uint32_t>(x.sorted_keys[it.pstart + k]) & 7u);
+        info = 0x400u;
+      } else if (it.pcount == 1) {
         const vx_primitive pr = x.prims[pidx];
         const Cell cell = unpack_cell(it.cell);
         if (vx_prim_shape(&pr) == VX_SHAPE_SPHERE && pr.r[0] <= kFloatMaskRadius) {
@@ -569,8 +554,16 @@ __global__ void __launch_bounds__(kBlock, MinBlocks) leafparent_kernel(Ctx x) {
         const uint64_t cell_bits = __shfl_sync(kFullMask, it.cell, src);
         const uint32_t pstart = __shfl_sync(kFullMask, it.pstart, src);
         const uint32_t pcount = __shfl_sync(kFullMask, it.pcount, src);
-        if (busy && !one_sphere)
-          mask = list_leaf_mask(x.prims, pairs + pstart, pcount, cell_bits, c, world_exp, mask);
+        const uint32_t src_touched = __shfl_sync(kFullMask, touched, src);
+        const bool sorted = (src_info & 0x400u) != 0;
+        const uint32_t n = one_sphere || !busy ? 0u : (sorted ? 1u : pcount);
+        for (uint32_t k = 0; k < n; ++k) {
+          const vx_primitive *pr =
+              x.prims + (sorted ? pstart + __popc(src_touched & ((1u << c) - 1u)) : pairs[pstart + k]);
+          const uint64_t m = sorted ? pr->r[0] | (static_cast<uint64_t>(pr->r[1]) << 32)
+                                    : other_leaf_mask(pr, cell_bits, c);
+          mask = vx_prim_op(pr) == VX_OP_ADD ? (mask | m) : (mask & ~m);
+        }
       }
       // An unchanged mask keeps its canonical ref: no probe of the leaf set.
       if (busy && mask != old_mask) {
@@ -1002,7 +995,7 @@ vx_status run_pipeline(vx_dag *d, const vx_primitive *prims,
                        uint32_t blocks_per_sm = 0 /* 0: the edit.blocks_per_sm knob */,
                        int small = -1 /* -1: by host_count as a primitive batch */,
                        const uint64_t *sorted_keys = nullptr /* EditCtx::sorted_keys */) {
-  Ctx x{d->t, d->a, prims, d_count, host_count};
+  Ctx x{d->t, d->a, prims, d_count, host_count, nullptr};
   EditCtx e{d->t.hdr, d->a, prims, d_count, host_count, d->t.depth,
             static_cast<uint32_t>(tune::get(tune::kEditBigItem)), nullptr};
   const uint32_t depth = d->t.depth;
@@ -1011,7 +1004,7 @@ vx_status run_pipeline(vx_dag *d, const vx_primitive *prims,
                                        : static_cast<uint32_t>(tune::get(tune::kEditBlocksPerSm)));
   if (!terrain && (small < 0 ? small_batch(host_count, false) : small != 0))
     return run_small(d, x, e, s);
-  e.sorted_keys = sorted_keys;
+  e.sorted_keys = x.sorted_keys = sorted_keys;
   if (sorted_keys != nullptr) e.big_item = 0xffffffffu; // no list is walked
   {
     prof::Scope sc("dag_init", s);
@@ -1033,15 +1026,10 @@ vx_status run_pipeline(vx_dag *d, const vx_primitive *prims,
             <<<level_grid(grid, l, kBlock), kBlock, 0, s>>>(e, tree, l);
     }
     VX_TRY_CUDA(cudaGetLastError());
-    if (sorted_keys != nullptr) continue;
+    if (sorted_keys != nullptr || terrain) continue; // no long lists
     {
       prof::Scope sc("dag_expand_big", s);
-      if (terrain)
-        expand_big_kernel<DagTree, true>
-            <<<level_grid(sm_count() * 2, l, 1), kBlock, 0, s>>>(e, tree, l);
-      else
-        expand_big_kernel<DagTree, false>
-            <<<level_grid(sm_count(), l, 1), kBigBlock, 0, s>>>(e, tree, l);
+      expand_long_kernel<DagTree><<<long_grid(l), kLongBlock, 0, s>>>(e, tree, l);
     }
     VX_TRY_CUDA(cudaGetLastError());
   }
@@ -1366,7 +1354,7 @@ vx_status vx_dag_apply_voxels(vx_dag *d, const vx_voxel *edits, uint32_t count,
   if (small_batch(count, true) &&
       plain_prep_layout(workspace, workspace_bytes, edits, count, op, 0, &prep)) {
     // one cooperative launch: voxels -> leaf masks -> the edit
-    Ctx x{d->t, d->a, prep.prims, prep.nprims, count};
+    Ctx x{d->t, d->a, prep.prims, prep.nprims, count, nullptr};
     const EditCtx e{d->t.hdr, d->a, prep.prims, prep.nprims, count, d->t.depth,
                     static_cast<uint32_t>(vx::tune::get(vx::tune::kEditBigItem)), nullptr};
     if (d->status_alias == nullptr) {

@@ -16,6 +16,10 @@
 #include "common.cuh"
 #include "voxel_b200_device.cuh"
 
+#include <cooperative_groups.h>
+
+#include <algorithm>
+
 namespace vx::edit {
 
 // Internal primitive shapes beyond the public sphere / box.
@@ -274,6 +278,20 @@ static __device__ __noinline__ uint32_t other_children(const vx_primitive *prim,
     }
   }
   return touched | (covered << 8);
+}
+
+// The voxels of leaf c of the 8^3 cell `cell` that any edit primitive covers
+// (a function of its own for the same reason).
+static __device__ __noinline__ uint64_t other_leaf_mask(const vx_primitive *prim, uint64_t cell,
+                                                        uint32_t c) {
+  const vx_primitive p = *prim;
+  const Cell k = unpack_cell(cell);
+  const int64_t ox = int64_t(2 * k.x + (c & 1u)) * 4;
+  const int64_t oy = int64_t(2 * k.y + ((c >> 1) & 1u)) * 4;
+  const int64_t oz = int64_t(2 * k.z + (c >> 2)) * 4;
+  const uint32_t cls = classify<false>(p, 0, ox, oy, oz, 4);
+  if (cls == VX_CELL_EMPTY) return 0ull;
+  return cls == VX_CELL_FULL ? ~0ull : leaf_mask<false>(p, 0, ox, oy, oz);
 }
 
 // One work item of the top-down expansion (32 bytes).  Two fields change
@@ -1065,19 +1083,13 @@ inline uint32_t level_grid(uint32_t grid, uint32_t l, uint32_t per_block) {
   return need < grid ? need : grid;
 }
 
-// Expansion of the long-list items of level l: one block of Threads
-// threads per item.  Three walks over the list: the last fully-covering
-// primitive per child (block max), the partial primitives after it per child
-// (block sum), then an order-preserving block-wide compaction of those into
-// each child's list.  The root of a batch carries every primitive and is
-// expanded by one block alone, so edits use a wide block (kBigBlock); the
-// terrain generator's classification needs more registers than a wide
-// block leaves a thread, so terrain builds use kBlock.  Lists of up to
-// kBigCache primitives are classified once: walk 1 keeps each primitive's
+// Expansion of the long-list items of level l inside the small cooperative
+// kernels: one block of Threads threads per item.  Three walks over the list:
+// the last fully-covering primitive per child (block max), the partial
+// primitives after it per child (block sum), then an order-preserving
+// block-wide compaction of those into each child's list.  Lists of up to
+// Cache primitives are classified once: walk 1 keeps each primitive's
 // per-child MIXED bits in shared memory for walks 2 and 3.
-constexpr uint32_t kBigBlock = 512;
-constexpr uint32_t kBigCache = 32768;
-
 template <class Policy, bool Terrain, uint32_t Threads, uint32_t Cache>
 __device__ __forceinline__ void expand_big_body(EditCtx x, Policy pol, uint32_t l, Blocks blk) {
   Header *h = x.hdr;
@@ -1270,10 +1282,264 @@ __device__ __forceinline__ void expand_big_body(EditCtx x, Policy pol, uint32_t 
   }
 }
 
-template <class Policy, bool Terrain, uint32_t Threads = Terrain ? kBlock : kBigBlock>
-__global__ void __launch_bounds__(Threads)
-    expand_big_kernel(EditCtx x, Policy pol, uint32_t l) {
-  expand_big_body<Policy, Terrain, Threads, kBigCache>(x, pol, l, launch_blocks());
+// The same for the batches' own launches.  A list longer than kLongList is
+// expanded by a cluster of eight blocks (the root of a batch carries every
+// primitive), a shorter one by one block.  Each warp owns a contiguous part
+// of the list, so its order is kept without a barrier per step: the three
+// walks are separated by one exchange each (the covering primitive per child,
+// the counts per warp and child, the room taken), over the blocks' shared
+// memory inside a cluster.  Classification treats a primitive's eight children
+// together and is kept as a byte per primitive for the later walks.
+// On B200, nine levels of two batches of 32,768 primitives: 1.18 -> 0.48 ms;
+// eleven levels of 16,384 spheres: 0.27 -> 0.14 ms.
+constexpr uint32_t kLongBlock = 512, kLongCluster = 8, kLongList = 4096;
+constexpr uint32_t kLongWarps = kLongBlock / kWarp;
+constexpr uint32_t kLongCache = 32768; // primitives per block whose bits are kept
+
+struct LongShared {
+  uint8_t mixed[kLongCache];
+  int32_t warp_last[kLongWarps][8];
+  uint32_t warp_count[kLongWarps][8]; // then each warp's offset in its block
+  int32_t last[kLongCluster][8];      // per block of the cluster
+  uint32_t count[kLongCluster][8];
+  uint32_t at[8];                     // first pair of each child's list
+  uint32_t room;
+  uint32_t failed[kLongCluster];
+};
+
+template <class Policy, uint32_t Cl>
+__device__ __forceinline__ void expand_long_item(const EditCtx &x, const Policy &pol, uint32_t l,
+                                                 uint32_t wi, uint32_t base, uint32_t next_base,
+                                                 LongShared &s) {
+  namespace cg = cooperative_groups;
+  cg::cluster_group cluster = cg::this_cluster();
+  const uint32_t rank = Cl > 1 ? cluster.block_rank() : 0u;
+  auto sync_all = [&]() {
+    if constexpr (Cl > 1) cluster.sync();
+    else __syncthreads();
+  };
+  // v into *field of every block of the cluster
+  auto share = [&](auto *field, auto v) {
+    if constexpr (Cl > 1) {
+      for (uint32_t r = 0; r < Cl; ++r) *cluster.map_shared_rank(field, r) = v;
+    } else {
+      *field = v;
+    }
+  };
+  Header *h = x.hdr;
+  const uint32_t t = threadIdx.x, lane = lane_id(), warp = t / kWarp;
+  const uint32_t *in_pairs = x.a.pairs[l & 1u];
+  uint32_t *out_pairs = x.a.pairs[(l + 1) & 1u];
+  const uint32_t csize = 4u << (x.depth - l - 1);
+  const Item it = x.a.items[base + wi];
+  const uint32_t units = (it.pcount + kWarp - 1) / kWarp;
+  const uint32_t part = (units + Cl * kLongWarps - 1) / (Cl * kLongWarps) * kWarp; // per warp
+  const uint32_t block_first = rank * kLongWarps * part;
+  const uint32_t first = min(block_first + warp * part, it.pcount);
+  const uint32_t end = min(first + part, it.pcount);
+  const bool cached = kLongWarps * part <= kLongCache;
+  const uint32_t old_child = rank == 0 && t < 8 ? pol.child(l, it.old, t) : 0u;
+  const Cell cell = unpack_cell(it.cell);
+  auto classify8 = [&](uint32_t p, uint32_t &touched, uint32_t &covered) {
+    const vx_primitive pr = x.prims[p];
+    if (vx_prim_shape(&pr) == VX_SHAPE_SPHERE && pr.r[0] < kFastRadius) {
+      sphere_classify_children(pr, cell.x * 2u * csize, cell.y * 2u * csize, cell.z * 2u * csize,
+                               csize, touched, covered);
+    } else {
+      const uint32_t tc = other_children(x.prims + p, it.cell, csize);
+      touched = tc & 0xffu;
+      covered = tc >> 8;
+    }
+  };
+  // Walk 1: the last covering primitive per child.
+  int32_t last[8];
+#pragma unroll
+  for (uint32_t c = 0; c < 8; ++c) last[c] = -1;
+  for (uint32_t k = first + lane; k < end; k += kWarp) {
+    const uint32_t p = in_pairs[it.pstart + k];
+    uint32_t touched, covered;
+    classify8(p, touched, covered);
+#pragma unroll
+    for (uint32_t c = 0; c < 8; ++c)
+      if ((covered >> c) & 1u) last[c] = static_cast<int32_t>(p); // lists ascend
+    if (cached) s.mixed[k - block_first] = static_cast<uint8_t>(touched & ~covered);
+  }
+#pragma unroll
+  for (uint32_t c = 0; c < 8; ++c) {
+    const int32_t m = __reduce_max_sync(kFullMask, last[c]);
+    if (lane == 0) s.warp_last[warp][c] = m;
+  }
+  __syncthreads();
+  if (t < 8) {
+    int32_t m = -1;
+    for (uint32_t w = 0; w < kLongWarps; ++w) m = max(m, s.warp_last[w][t]);
+    share(&s.last[rank][t], m);
+  }
+  sync_all();
+#pragma unroll
+  for (uint32_t c = 0; c < 8; ++c) {
+    last[c] = s.last[0][c];
+    for (uint32_t r = 1; r < Cl; ++r) last[c] = max(last[c], s.last[r][c]);
+  }
+  // The children that entry k goes down to (bit c), and its primitive.
+  auto goes_down = [&](uint32_t k, uint32_t &p) {
+    if (k >= end) return 0u;
+    p = in_pairs[it.pstart + k];
+    uint32_t mixed, covered;
+    if (cached) {
+      mixed = s.mixed[k - block_first]; // the warp wrote it
+    } else {
+      classify8(p, mixed, covered);
+      mixed &= ~covered;
+    }
+    uint32_t keep = 0;
+#pragma unroll
+    for (uint32_t c = 0; c < 8; ++c)
+      if (static_cast<int32_t>(p) > last[c]) keep |= 1u << c;
+    return keep & mixed;
+  };
+  // Walk 2: how many go down, per warp and child (lane c counts child c).
+  uint32_t cnt = 0;
+  for (uint32_t k0 = first; k0 < end; k0 += kWarp) {
+    uint32_t p = 0;
+    const uint32_t keep = goes_down(k0 + lane, p);
+#pragma unroll
+    for (uint32_t c = 0; c < 8; ++c) {
+      const uint32_t b = __ballot_sync(kFullMask, (keep >> c) & 1u);
+      if (lane == c) cnt += __popc(b);
+    }
+  }
+  if (lane < 8) s.warp_count[warp][lane] = cnt;
+  __syncthreads();
+  if (t < 8) {
+    uint32_t run = 0;
+    for (uint32_t w = 0; w < kLongWarps; ++w) {
+      const uint32_t v = s.warp_count[w][t];
+      s.warp_count[w][t] = run;
+      run += v;
+    }
+    share(&s.count[rank][t], run);
+  }
+  sync_all();
+  // Block 0's first lanes take the room and write the children (lane c child c).
+  if (rank == 0 && warp == 0) {
+    const uint32_t c = lane & 7u;
+    uint32_t total = 0;
+    for (uint32_t r = 0; r < Cl; ++r) total += s.count[r][c];
+    int32_t lf = s.last[0][c];
+    for (uint32_t r = 1; r < Cl; ++r) lf = max(lf, s.last[r][c]);
+    const int64_t oz = int64_t(2 * cell.z + (c >> 2)) * csize;
+    const uint32_t cv = lf >= 0 ? pol.const_value(x.prims[lf], oz, csize) : 0u;
+    uint32_t inc = total;
+#pragma unroll
+    for (uint32_t d = 1; d < 8; d <<= 1) {
+      const uint32_t o = __shfl_up_sync(kFullMask, inc, d, 8);
+      if (c >= d) inc += o;
+    }
+    const uint32_t np = __shfl_sync(kFullMask, inc, 7);
+    const uint32_t cm =
+        __ballot_sync(kFullMask, total != 0 || (Policy::kItemsForConst && lf >= 0)) & 0xffu;
+    const uint32_t km = __ballot_sync(kFullMask, lf >= 0) & 0xffu;
+    const uint32_t kf = __ballot_sync(kFullMask, lf >= 0 && cv == 1u) & 0xffu;
+    const uint32_t ni = __popc(cm);
+    uint32_t item_at = 0, pair_at = 0, room = 1;
+    if (lane == 0) {
+      if (ni) item_at = atomicAdd(&h->item_count[l + 1], ni);
+      if (np) pair_at = atomicAdd(&h->pair_count[l + 1], np);
+      // this item's own room (an overflow elsewhere fails the edit at the
+      // next stage; writing within the buffers meanwhile is harmless)
+      if (ni && uint64_t(next_base) + item_at + ni > x.a.item_cap) room = 0;
+      if (np && uint64_t(pair_at) + np > x.a.pair_cap) room = 0;
+      if (!room) set_status(&h->status, kDevCapacity);
+      Item &me = x.a.items[base + wi]; // every thread holds its own copy
+      me.child_base = next_base + item_at;
+      me.masks = cm | (km << 8) | (kf << 16);
+      me.pstart = ni;
+    }
+    item_at = __shfl_sync(kFullMask, item_at, 0);
+    pair_at = __shfl_sync(kFullMask, pair_at, 0);
+    room = __shfl_sync(kFullMask, room, 0);
+    if (lane < 8 && room) {
+      if (lf >= 0) pol.replaced(l, it.old, c);
+      if ((cm >> c) & 1u) {
+        Item ci{};
+        ci.cell = child_cell(it.cell, c);
+        ci.old = lf >= 0 ? cv : old_child;
+        ci.pstart = pair_at + inc - total;
+        ci.pcount = total;
+        ci.result = base + wi;
+        const uint32_t k = item_at + __popc(cm & ((1u << c) - 1u));
+        x.a.items[next_base + k] = ci;
+        note_big(x, l + 1, k, total);
+      }
+    }
+    if (lane < 8) share(&s.at[c], pair_at + inc - total);
+    if (lane == 0) share(&s.room, room);
+  }
+  sync_all();
+  // Walk 3: each warp appends its part, in order (lane c holds child c's next
+  // place).
+  if (s.room) {
+    uint32_t to = 0;
+    if (lane < 8) {
+      to = s.at[lane] + s.warp_count[warp][lane];
+      if constexpr (Cl > 1)
+        for (uint32_t r = 0; r < rank; ++r) to += s.count[r][lane];
+    }
+    for (uint32_t k0 = first; k0 < end; k0 += kWarp) {
+      uint32_t p = 0;
+      const uint32_t keep = goes_down(k0 + lane, p);
+#pragma unroll
+      for (uint32_t c = 0; c < 8; ++c) {
+        const uint32_t b = __ballot_sync(kFullMask, (keep >> c) & 1u);
+        const uint32_t at = __shfl_sync(kFullMask, to, c);
+        if ((keep >> c) & 1u) out_pairs[at + __popc(b & lanemask_lt())] = p;
+        if (lane == c) to += __popc(b);
+      }
+    }
+  }
+  sync_all(); // the buffers are reused, or the blocks end, only when all are done
+}
+
+template <class Policy>
+__global__ void __cluster_dims__(kLongCluster, 1, 1) __launch_bounds__(kLongBlock, 1)
+    expand_long_kernel(EditCtx x, Policy pol, uint32_t l) {
+  namespace cg = cooperative_groups;
+  __shared__ LongShared s;
+  cg::cluster_group cluster = cg::this_cluster();
+  Header *h = x.hdr;
+  const uint32_t nbig = min(h->big_count[l], x.a.big_cap / 2u);
+  const uint32_t *bigs = big_list(x.a, l);
+  const uint32_t base = h->item_off[l];
+  const uint32_t next_base = base + h->item_count[l];
+  // A failed edit: the blocks of a cluster leave together or not at all (one
+  // may see a failure that another has not seen yet).
+  const uint32_t failed = edit_failed(h) ? 1u : 0u;
+  cluster.sync(); // every block has started: its shared memory may be written
+  if (threadIdx.x < kLongCluster)
+    *cluster.map_shared_rank(&s.failed[cluster.block_rank()], threadIdx.x) = failed;
+  cluster.sync();
+  uint32_t any = 0;
+  for (uint32_t r = 0; r < kLongCluster; ++r) any |= s.failed[r];
+  if (any) {
+    cluster.sync(); // no block ends while another may still write to it
+    return;
+  }
+  const uint32_t clusters = gridDim.x / kLongCluster;
+  for (uint32_t b = blockIdx.x / kLongCluster; b < nbig; b += clusters)
+    if (x.a.items[base + bigs[b]].pcount > kLongList)
+      expand_long_item<Policy, kLongCluster>(x, pol, l, bigs[b], base, next_base, s);
+  for (uint32_t b = blockIdx.x; b < nbig; b += gridDim.x)
+    if (x.a.items[base + bigs[b]].pcount <= kLongList)
+      expand_long_item<Policy, 1>(x, pol, l, bigs[b], base, next_base, s);
+  cluster.sync(); // (a block's last exchange may still be read by its neighbours)
+}
+
+// Blocks of expand_long_kernel for level l: a cluster per item of the level,
+// at most a block per SM.
+inline uint32_t long_grid(uint32_t l) {
+  const uint32_t most = static_cast<uint32_t>(sm_count()) / kLongCluster * kLongCluster;
+  return std::max(kLongCluster, level_grid(most, l, 1) / kLongCluster * kLongCluster);
 }
 
 } // namespace vx::edit
