@@ -107,25 +107,45 @@ __device__ __forceinline__ uint64_t vx_dag_get_leaf(const vx_dag_view &v, uint32
  * coordinates are floor(origin + t dir) kept inside the cell and never moving
  * against the ray.  Each step advances one coordinate, so at most
  * 3 * world steps run. */
-__device__ inline vx_ray_hit vx_dag_raycast(const vx_dag_view &v, const vx_ray &ray) {
-  vx_ray_hit miss;
-  miss.voxel[0] = miss.voxel[1] = miss.voxel[2] = ~0u;
-  miss.face = VX_FACE_NO_HIT;
-  miss.t = -1.0f;
-  const uint32_t D = v.depth;
-  const int32_t W = 4 << D;
+__device__ __forceinline__ vx_ray_hit vx_ray_miss() {
+  vx_ray_hit m;
+  m.voxel[0] = m.voxel[1] = m.voxel[2] = ~0u;
+  m.face = VX_FACE_NO_HIT;
+  m.t = -1.0f;
+  return m;
+}
+
+/* A ray under way (vx_dag_ray_begin, then vx_dag_ray_step until it ends).
+ * path[k * path_stride] = ref of the level-k cell holding the current voxel,
+ * valid for k <= l: depth + 1 words that the caller provides (a local array,
+ * or a column of shared memory).  A step keeps the cells that still hold the
+ * next voxel, so the walk resumes below the deepest common cell instead of at
+ * the root. */
+struct vx_dag_ray {
+  float o[3], d[3], inv[3];
+  float t, t_max;
+  int32_t vox[3];
+  uint32_t face, l, step;
+};
+
+/* Clips the ray to the world; false: it misses the world (no hit). */
+__device__ __forceinline__ bool vx_dag_ray_begin(const vx_dag_view &v, const vx_ray &ray,
+                                                 vx_dag_ray &s, uint32_t *path) {
+  const int32_t W = 4 << v.depth;
   const float Wf = (float)W;
-  const float o[3] = {ray.origin[0], ray.origin[1], ray.origin[2]};
-  const float d[3] = {ray.dir[0], ray.dir[1], ray.dir[2]};
   float t0 = 0.0f, t1 = __int_as_float(0x7f800000);
   int entry = -1;
+  s.t_max = ray.t_max;
+#pragma unroll
   for (int a = 0; a < 3; ++a) {
-    if (d[a] == 0.0f) {
-      if (!(o[a] >= 0.0f && o[a] < Wf)) return miss;
+    const float o = s.o[a] = ray.origin[a], d = s.d[a] = ray.dir[a];
+    s.inv[a] = __frcp_rn(d);
+    if (d == 0.0f) {
+      if (!(o >= 0.0f && o < Wf)) return false;
       continue;
     }
-    const float ta = __fdiv_rn(__fsub_rn(0.0f, o[a]), d[a]);
-    const float tb = __fdiv_rn(__fsub_rn(Wf, o[a]), d[a]);
+    const float ta = __fdiv_rn(__fsub_rn(0.0f, o), d);
+    const float tb = __fdiv_rn(__fsub_rn(Wf, o), d);
     const float tn = ta < tb ? ta : tb, tf = ta < tb ? tb : ta;
     if (tn > t0) {
       t0 = tn;
@@ -133,88 +153,133 @@ __device__ inline vx_ray_hit vx_dag_raycast(const vx_dag_view &v, const vx_ray &
     }
     if (tf < t1) t1 = tf;
   }
-  if (!(t0 < t1) || !(t0 <= ray.t_max)) return miss;
-  int32_t vox[3];
+  if (!(t0 < t1) || !(t0 <= ray.t_max)) return false;
+  s.face = 0u;
+#pragma unroll
   for (int a = 0; a < 3; ++a) {
     if (a == entry) {
-      vox[a] = d[a] > 0.0f ? 0 : W - 1;
+      s.vox[a] = s.d[a] > 0.0f ? 0 : W - 1;
+      s.face = s.d[a] > 0.0f ? 2u * a + 1u : 2u * a;
     } else {
-      float f = floorf(__fadd_rn(o[a], __fmul_rn(t0, d[a])));
+      float f = floorf(__fadd_rn(s.o[a], __fmul_rn(t0, s.d[a])));
       f = f < 0.0f ? 0.0f : (f > Wf - 1.0f ? Wf - 1.0f : f);
-      vox[a] = (int32_t)f;
+      s.vox[a] = (int32_t)f;
     }
   }
-  uint32_t face = entry < 0 ? 0u : (d[entry] > 0.0f ? 2u * entry + 1u : 2u * entry);
-  float t = t0;
-  /* path[k] = ref of the level-k cell holding the current voxel, valid for
-   * k <= l; a step keeps the cells that still hold the next voxel, so the
-   * walk resumes below the deepest common cell instead of at the root. */
-  uint32_t path[15]; /* depth <= 14 */
+  s.t = t0;
   path[0] = *v.root;
-  uint32_t l = 0;
-  const uint32_t limit = 3u * (uint32_t)W + 8u;
-  for (uint32_t step = 0; step < limit; ++step) {
-    uint32_t ref = path[l];
-    for (; l < D && ref >= 2u; ++l) {
-      const uint32_t sh = D + 1 - l;
-      const uint32_t c = (((uint32_t)vox[0] >> sh) & 1u) | ((((uint32_t)vox[1] >> sh) & 1u) << 1) |
-                         ((((uint32_t)vox[2] >> sh) & 1u) << 2);
-      ref = vx_dag_item_child(v.pool[l] + (ref - 2u), c);
-      path[l + 1] = ref;
-    }
-    int32_t side;
-    if (ref == 1u) {
-      side = 0;
-    } else if (ref >= 2u) {
-      const uint32_t bit = (vox[0] & 3) + 4u * (vox[1] & 3) + 16u * (vox[2] & 3);
-      side = ((v.leaves[ref - 2u] >> bit) & 1ull) ? 0 : 1;
-    } else {
-      side = 4 << (D - l);
-    }
-    if (side == 0) {
-      vx_ray_hit h;
-      h.voxel[0] = (uint32_t)vox[0];
-      h.voxel[1] = (uint32_t)vox[1];
-      h.voxel[2] = (uint32_t)vox[2];
-      h.face = face;
-      h.t = t;
-      return h;
-    }
-    int32_t cmin[3];
-    for (int a = 0; a < 3; ++a) cmin[a] = vox[a] & ~(side - 1);
-    float tx = 0.0f;
-    int ax = -1;
+  s.l = 0;
+  s.step = 0;
+  return true;
+}
+
+/* One step: walk to the cell that holds the current voxel, end there (true:
+ * *hit is the result, a hit or a miss) or move on to the next voxel.  The side
+ * that the ray leaves the cell by has the smallest quotient (b - o) / d.  A
+ * product with the reciprocal is within 2^-21 of the quotient, so when the
+ * smallest product is clear of the others by more than that, only its
+ * quotient is divided out; otherwise all three are. */
+__device__ __forceinline__ bool vx_dag_ray_step(const vx_dag_view &v, vx_dag_ray &s,
+                                                uint32_t *path, uint32_t path_stride,
+                                                vx_ray_hit *hit) {
+  const uint32_t D = v.depth;
+  const int32_t W = 4 << D;
+  uint32_t l = s.l;
+  uint32_t ref = path[l * path_stride];
+  for (; l < D && ref >= 2u; ++l) {
+    const uint32_t sh = D + 1 - l;
+    const uint32_t c = (((uint32_t)s.vox[0] >> sh) & 1u) | ((((uint32_t)s.vox[1] >> sh) & 1u) << 1) |
+                       ((((uint32_t)s.vox[2] >> sh) & 1u) << 2);
+    ref = vx_dag_item_child(v.pool[l] + (ref - 2u), c);
+    path[(l + 1) * path_stride] = ref;
+  }
+  int32_t side;
+  if (ref == 1u) {
+    side = 0;
+  } else if (ref >= 2u) {
+    const uint32_t bit = (s.vox[0] & 3) + 4u * (s.vox[1] & 3) + 16u * (s.vox[2] & 3);
+    side = ((v.leaves[ref - 2u] >> bit) & 1ull) ? 0 : 1;
+  } else {
+    side = 4 << (D - l);
+  }
+  if (side == 0) {
+    hit->voxel[0] = (uint32_t)s.vox[0];
+    hit->voxel[1] = (uint32_t)s.vox[1];
+    hit->voxel[2] = (uint32_t)s.vox[2];
+    hit->face = s.face;
+    hit->t = s.t;
+    return true;
+  }
+  *hit = vx_ray_miss();
+  int32_t cmin[3];
+  float gap[3], est[3];
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    cmin[a] = s.vox[a] & ~(side - 1);
+    gap[a] = __fsub_rn((float)(s.d[a] > 0.0f ? cmin[a] + side : cmin[a]), s.o[a]);
+    est[a] = s.d[a] == 0.0f ? 3.0e38f : __fmul_rn(gap[a], s.inv[a]);
+  }
+  int ax = est[1] < est[0] ? 1 : 0;
+  if (est[2] < est[ax]) ax = 2;
+  const float least = ax == 0 ? est[0] : (ax == 1 ? est[1] : est[2]);
+  const float o1 = ax == 0 ? est[1] : est[0], o2 = ax == 2 ? est[1] : est[2];
+  float tx;
+  /* (false when any of the three is infinite or NaN) */
+  if (o1 - least > 1.0e-6f * (fabsf(o1) + fabsf(least)) + 1.0e-30f &&
+      o2 - least > 1.0e-6f * (fabsf(o2) + fabsf(least)) + 1.0e-30f) {
+    tx = __fdiv_rn(ax == 0 ? gap[0] : (ax == 1 ? gap[1] : gap[2]),
+                   ax == 0 ? s.d[0] : (ax == 1 ? s.d[1] : s.d[2]));
+  } else {
+    tx = 0.0f;
+    ax = -1;
+#pragma unroll
     for (int a = 0; a < 3; ++a) {
-      if (d[a] == 0.0f) continue;
-      const float b = (float)(d[a] > 0.0f ? cmin[a] + side : cmin[a]);
-      const float ta = __fdiv_rn(__fsub_rn(b, o[a]), d[a]);
+      if (s.d[a] == 0.0f) continue;
+      const float ta = __fdiv_rn(gap[a], s.d[a]);
       if (ax < 0 || ta < tx) {
         tx = ta;
         ax = a;
       }
     }
-    if (ax < 0 || !(tx <= ray.t_max)) return miss;
-    const int32_t nv = d[ax] > 0.0f ? cmin[ax] + side : cmin[ax] - 1;
-    if (nv < 0 || nv >= W) return miss;
-    uint32_t moved = (uint32_t)(vox[ax] ^ nv);
-    for (int b = 0; b < 3; ++b) {
-      if (b == ax || d[b] == 0.0f) continue;
-      const float lo = (float)(d[b] > 0.0f ? vox[b] : cmin[b]);
-      const float hi = (float)(d[b] > 0.0f ? cmin[b] + side - 1 : vox[b]);
-      float f = floorf(__fadd_rn(o[b], __fmul_rn(tx, d[b])));
-      f = f < lo ? lo : (f > hi ? hi : f);
-      moved |= (uint32_t)(vox[b] ^ (int32_t)f);
-      vox[b] = (int32_t)f;
-    }
-    vox[ax] = nv;
-    /* The level-k cell (side 2^(D+2-k)) still holds the voxel iff no
-     * coordinate bit at or above D + 2 - k changed. */
-    const uint32_t keep = D + 1u - (31u - (uint32_t)__clz((int)moved));
-    if (keep < l) l = keep;
-    t = tx;
-    face = d[ax] > 0.0f ? 2u * ax + 1u : 2u * ax;
+    if (ax < 0) return true;
   }
-  return miss;
+  if (!(tx <= s.t_max)) return true;
+  uint32_t moved = 0;
+#pragma unroll
+  for (int b = 0; b < 3; ++b) {
+    int32_t nv;
+    if (b == ax) {
+      nv = s.d[b] > 0.0f ? cmin[b] + side : cmin[b] - 1;
+      if (nv < 0 || nv >= W) return true;
+      s.face = s.d[b] > 0.0f ? 2u * b + 1u : 2u * b;
+    } else if (s.d[b] == 0.0f) {
+      continue;
+    } else {
+      const float lo = (float)(s.d[b] > 0.0f ? s.vox[b] : cmin[b]);
+      const float hi = (float)(s.d[b] > 0.0f ? cmin[b] + side - 1 : s.vox[b]);
+      float f = floorf(__fadd_rn(s.o[b], __fmul_rn(tx, s.d[b])));
+      f = f < lo ? lo : (f > hi ? hi : f);
+      nv = (int32_t)f;
+    }
+    moved |= (uint32_t)(s.vox[b] ^ nv);
+    s.vox[b] = nv;
+  }
+  /* The level-k cell (side 2^(D+2-k)) still holds the voxel iff no
+   * coordinate bit at or above D + 2 - k changed. */
+  const uint32_t keep = D + 1u - (31u - (uint32_t)__clz((int)moved));
+  s.l = keep < l ? keep : l;
+  s.t = tx;
+  return ++s.step >= 3u * (uint32_t)W + 8u;
+}
+
+__device__ inline vx_ray_hit vx_dag_raycast(const vx_dag_view &v, const vx_ray &ray) {
+  vx_ray_hit hit = vx_ray_miss();
+  vx_dag_ray s;
+  uint32_t path[15]; /* depth <= 14 */
+  if (!vx_dag_ray_begin(v, ray, s, path)) return hit;
+  while (!vx_dag_ray_step(v, s, path, 1u, &hit)) {
+  }
+  return hit;
 }
 
 /* ------------------------------------------------------------------ SVO -- */

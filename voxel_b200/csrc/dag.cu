@@ -746,11 +746,51 @@ __global__ void query_kernel(vx_dag_view v, const vx_voxel *pts, uint32_t n,
   out[i] = vx_dag_get_voxel(v, p.x, p.y, p.z);
 }
 
-__global__ void raycast_kernel(vx_dag_view v, const vx_ray *rays, uint32_t n,
-                               vx_ray_hit *hits) {
-  const uint64_t i = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x;
-  if (i >= n) return;
-  hits[i] = vx_dag_raycast(v, rays[i]);
+// Rays differ in length by orders of magnitude (a miss of the world, a ray
+// along a cave), so a thread per ray leaves a warp waiting for its longest:
+// 5.75 of 32 lanes were active per instruction.  A warp owns per_warp rays
+// instead, and lanes whose ray has ended take the next ones once kRayRefill
+// of them are idle.  The cells that a ray's path goes through are kept in a
+// column of shared memory per thread.  1 M rays (half downwards on the
+// terrain, half at random) on a 4096^3 DAG, B200: 0.86 -> 0.65 ms, now bound
+// by the longest rays (65,536 rays alone take 0.32 ms): refills of 16 lanes
+// take 0.69 ms, 8 steps between refills 0.78 ms, two or three times as many
+// warps 0.77-0.83 ms, walks of at most 1-3 levels a step 0.75-0.93 ms.
+constexpr uint32_t kRayRefill = 8, kRaySteps = 4, kRayBlocksPerSm = 5;
+
+__global__ void __launch_bounds__(kBlock, kRayBlocksPerSm)
+    raycast_kernel(vx_dag_view v, const vx_ray *rays, uint32_t n, vx_ray_hit *hits,
+                   uint32_t per_warp) {
+  __shared__ uint32_t s_path[kMaxDepth + 1][kBlock];
+  uint32_t *path = &s_path[0][threadIdx.x];
+  const uint64_t warp = (blockIdx.x * uint64_t(kBlock) + threadIdx.x) / kWarp;
+  const uint64_t end = min(static_cast<uint64_t>(n), (warp + 1) * per_warp);
+  uint64_t next = warp * per_warp; // the same on the warp's lanes
+  vx_dag_ray ray;
+  uint32_t mine = 0;
+  bool active = false;
+  for (;;) {
+    const uint32_t idle = __ballot_sync(kFullMask, !active);
+    if (next < end && __popc(idle) >= kRayRefill) {
+      const uint64_t take = next + __popc(idle & lanemask_lt());
+      if (!active && take < end) {
+        mine = static_cast<uint32_t>(take);
+        active = vx_dag_ray_begin(v, rays[mine], ray, path);
+        if (!active) hits[mine] = vx_ray_miss();
+      }
+      next += __popc(idle);
+    } else if (idle == kFullMask) {
+      return; // no ray left
+    }
+    for (uint32_t k = 0; k < kRaySteps && active; ++k) {
+      vx_ray_hit hit;
+      if (vx_dag_ray_step(v, ray, path, kBlock, &hit)) {
+        hits[mine] = hit;
+        active = false;
+      }
+    }
+    __syncwarp();
+  }
 }
 
 __global__ void read_leaves_kernel(vx_dag_view v, uint32_t lx0, uint32_t ly0, uint32_t lz0,
@@ -1477,7 +1517,12 @@ vx_status vx_dag_raycast(const vx_dag *d, const vx_ray *rays, uint32_t count,
   vx::prof::Scope sc("dag_raycast", s);
   vx_dag_view view;
   VX_TRY(vx_dag_device_view(d, &view));
-  raycast_kernel<<<vx::ceil_div(count, kBlock), kBlock, 0, s>>>(view, rays, count, hits);
+  // As many warps as are resident at once, 32 rays each at least.
+  const uint32_t warps =
+      static_cast<uint32_t>(vx::sm_count()) * kRayBlocksPerSm * (kBlock / vx::kWarp);
+  const uint32_t per_warp = std::max(vx::kWarp, vx::ceil_div(count, warps));
+  const uint32_t blocks = vx::ceil_div(vx::ceil_div(count, per_warp), kBlock / vx::kWarp);
+  raycast_kernel<<<blocks, kBlock, 0, s>>>(view, rays, count, hits, per_warp);
   return vx::from_cuda(cudaGetLastError());
 }
 
