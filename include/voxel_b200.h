@@ -108,7 +108,7 @@ vx_status vx_scan_exclusive_sum_u64(uint64_t *data, uint32_t count,
  * the scan (a fixed device-memory budget, or code that must not call
  * cudaMalloc / cudaFree because they synchronise the device).  No counterpart
  * in the reference: its scans always take a caller workspace.  The scratch is
- * a 256 KiB array inside this library on each device, so count must be at
+ * a 272 KiB array inside this library on each device, so count must be at
  * most 2^28 (larger counts return VX_ERR_CAPACITY and touch nothing); calls
  * that can overlap on the GPU share that array and race; the first call in a
  * CUDA context (again after a device reset) looks up the array's address and

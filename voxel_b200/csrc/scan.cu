@@ -25,14 +25,24 @@ namespace scan {
 
 namespace {
 
-template <class T> typename RecordsFor<T>::type make_records(const ScanLayout &ws) {
+inline uint32_t groups_of(uint32_t tiles) { return ceil_div(tiles, kGroup); }
+
+// The records of `tiles` tiles: u32 sums keep a word per tile and two per
+// group in a row, u64 sums three arrays.  *end: the first byte after what a
+// call has to clear.
+template <class T>
+typename RecordsFor<T>::type make_records(const ScanLayout &ws, uint32_t tiles, char **end) {
   typename RecordsFor<T>::type r;
   if constexpr (sizeof(T) == 4) {
-    r.rec = ws.rec_a;
+    r.tile = ws.rec_a;
+    r.group_sum = r.tile + tiles;
+    r.group_inc = r.group_sum + groups_of(tiles);
+    *end = reinterpret_cast<char *>(r.group_inc + groups_of(tiles));
   } else {
     r.agg = ws.rec_a;
     r.inc = ws.rec_b;
     r.state = ws.rec_state;
+    *end = reinterpret_cast<char *>(ws.rec_state + tiles);
   }
   return r;
 }
@@ -40,12 +50,11 @@ template <class T> typename RecordsFor<T>::type make_records(const ScanLayout &w
 // One tile per block, tiles taken in the order of a global counter (a tile
 // only waits on tiles already taken by running blocks).  A full, aligned tile
 // arrives by one bulk copy; the last, partial tile and unaligned data use
-// guarded loads.  Pass 1 reads the rows from shared memory for per-row warp
-// totals, warp 0 scans the block and looks back, pass 2 re-reads the rows,
-// recomputes each thread's offset inside its warp (cheaper than holding it in
-// registers, which bound the resident blocks) and writes the prefix sums
-// straight to global memory.
-template <class T, bool Inclusive, bool Vectorised, class S = TileShape<T>>
+// guarded loads.  Each warp owns a contiguous part of the tile: it sums its
+// rows, the tile's sum is published at once, and while warp 0 looks back the
+// rows are scanned (32 lanes' vectors a row); then the rows are read from
+// shared memory again and the prefix sums written straight to global memory.
+template <class T, bool Inclusive, bool Vectorised, class S = Tile32<T>>
 __global__ void __launch_bounds__(S::kBlock, S::kMinBlocks)
     scan_kernel(T *__restrict__ data, uint32_t count, ScanLayout ws,
                 typename RecordsFor<T>::type records) {
@@ -53,8 +62,7 @@ __global__ void __launch_bounds__(S::kBlock, S::kMinBlocks)
   __shared__ __align__(128) T s_data[S::kTile];
   __shared__ uint64_t s_bar;
   __shared__ uint32_t s_tile;
-  __shared__ T s_warp[S::kWarps][S::kRows];
-  __shared__ T s_row_off[S::kRows];
+  __shared__ T s_warp[S::kWarps];
   __shared__ T s_prefix;
 
   const uint32_t t = threadIdx.x;
@@ -85,61 +93,74 @@ __global__ void __launch_bounds__(S::kBlock, S::kMinBlocks)
       s_data[i] = base + i < count ? data[base + i] : T(0);
     __syncthreads();
   }
-  const uint4 *rows = reinterpret_cast<const uint4 *>(s_data);
+  const uint32_t first_vec = warp * S::kRows * kWarp + lane; // row r: first_vec + 32 r
+  const uint4 *vecs = reinterpret_cast<const uint4 *>(s_data);
 
-  // Pass 1: per-row warp totals.
-#pragma unroll 4
+  // The lane's sum in each row, and the tile's sum.
+  T at[S::kRows];
+  T total = 0;
+#pragma unroll
   for (uint32_t r = 0; r < S::kRows; ++r) {
-    const uint4 q = rows[r * S::kBlock + t];
+    const uint4 q = vecs[first_vec + r * kWarp];
     const T *qt = reinterpret_cast<const T *>(&q);
     T sum = 0;
 #pragma unroll
     for (uint32_t e = 0; e < S::kPerVec; ++e) sum += qt[e];
-    sum = warp_sum<T>(sum);
-    if (lane == 0) s_warp[warp][r] = sum;
+    at[r] = sum;
+    total += sum;
   }
+  total = warp_sum<T>(total);
+  if (lane == 0) s_warp[warp] = total;
   __syncthreads();
-
-  if (warp == 0) {
-    T acc = 0;
+  T aggregate = 0, run = 0; // of the tile, of the warps before this one
 #pragma unroll
-    for (uint32_t r = 0; r < S::kRows; ++r) {
-      const T w = lane < S::kWarps ? s_warp[lane][r] : T(0);
-      const T wi = warp_inclusive_sum<T>(w);
-      if (lane < S::kWarps) s_warp[lane][r] = wi - w; // exclusive warp offset
-      if (lane == 0) s_row_off[r] = acc;
-      acc += __shfl_sync(kFullMask, wi, S::kWarps - 1);
-    }
-    const T prefix = warp_lookback<T>(records, tile, acc, ws.status);
+  for (uint32_t w = 0; w < S::kWarps; ++w) {
+    const T v = s_warp[w];
+    if (w < warp) run += v;
+    aggregate += v;
+  }
+  if (t == 0) {
+    if constexpr (sizeof(T) == 4) publish_group(records, tile, aggregate);
+    else records.publish(tile, tile == 0 ? kInclusive : kAggregate, aggregate);
+  }
+  if (warp == 0) {
+    T prefix;
+    if constexpr (sizeof(T) == 4) prefix = group_lookback(records, tile, aggregate, ws.status);
+    else prefix = warp_lookback<T>(records, tile, aggregate, ws.status);
     if (lane == 0) s_prefix = prefix;
   }
+  // Each lane's offset in the tile, row by row.
+#pragma unroll
+  for (uint32_t r = 0; r < S::kRows; ++r) {
+    const T inc = warp_inclusive_sum<T>(at[r]);
+    const T row = __shfl_sync(kFullMask, inc, kWarp - 1);
+    at[r] = run + inc - at[r];
+    run += row;
+  }
   __syncthreads();
 
-  // Pass 2: prefix sums, written straight to global memory.
+  // Prefix sums, written straight to global memory.
   const T tile_prefix = s_prefix;
-#pragma unroll 4
-  for (uint32_t r = 0; r < S::kRows; ++r) {
-    uint4 q = rows[r * S::kBlock + t];
-    T *qt = reinterpret_cast<T *>(&q);
-    T sum = 0;
 #pragma unroll
-    for (uint32_t e = 0; e < S::kPerVec; ++e) sum += qt[e];
-    T run = tile_prefix + s_row_off[r] + s_warp[warp][r] + (warp_inclusive_sum<T>(sum) - sum);
+  for (uint32_t r = 0; r < S::kRows; ++r) {
+    uint4 q = vecs[first_vec + r * kWarp];
+    T *qt = reinterpret_cast<T *>(&q);
+    T x = tile_prefix + at[r];
 #pragma unroll
     for (uint32_t e = 0; e < S::kPerVec; ++e) {
-      const T x = qt[e];
+      const T v = qt[e];
       if (Inclusive) {
-        run += x;
-        qt[e] = run;
+        x += v;
+        qt[e] = x;
       } else {
-        qt[e] = run;
-        run += x;
+        qt[e] = x;
+        x += v;
       }
     }
     if (bulk) {
-      reinterpret_cast<uint4 *>(data + base)[r * S::kBlock + t] = q;
+      reinterpret_cast<uint4 *>(data + base)[first_vec + r * kWarp] = q;
     } else {
-      const uint64_t i0 = base + (static_cast<uint64_t>(r) * S::kBlock + t) * S::kPerVec;
+      const uint64_t i0 = base + static_cast<uint64_t>(first_vec + r * kWarp) * S::kPerVec;
 #pragma unroll
       for (uint32_t e = 0; e < S::kPerVec; ++e)
         if (i0 + e < count) data[i0 + e] = qt[e];
@@ -147,35 +168,108 @@ __global__ void __launch_bounds__(S::kBlock, S::kMinBlocks)
   }
 }
 
+// Up to 64 KB of data: one block holds it in registers, with no records, so
+// nothing is cleared first (a launch instead of a memset and a launch:
+// 10,007 u32 10.6 -> 8.2 us of back-to-back calls on B200).
+constexpr uint32_t kSmallBlock = 512, kSmallRows = 8;
+template <class T> constexpr uint32_t small_max() {
+  return kSmallBlock * kSmallRows * (16u / sizeof(T));
+}
+
+template <class T, bool Inclusive, bool Vectorised>
+__global__ void __launch_bounds__(kSmallBlock)
+    scan_small_kernel(T *__restrict__ data, uint32_t count, uint32_t *status) {
+  constexpr uint32_t kPerVec = 16 / sizeof(T), kWarps = kSmallBlock / kWarp;
+  __shared__ T s_warp[kWarps];
+  const uint32_t t = threadIdx.x, lane = lane_id(), warp = t / kWarp;
+  if (t == 0) *status = kDevOk;
+  T v[kSmallRows][kPerVec], at[kSmallRows], run = 0;
+  const uint32_t first = (warp * kSmallRows * kWarp + lane) * kPerVec;
+#pragma unroll
+  for (uint32_t r = 0; r < kSmallRows; ++r) {
+    const uint32_t i = first + r * kWarp * kPerVec;
+    if (Vectorised && i + kPerVec <= count) {
+      const uint4 q = reinterpret_cast<const uint4 *>(data)[i / kPerVec];
+      const T *qt = reinterpret_cast<const T *>(&q);
+#pragma unroll
+      for (uint32_t e = 0; e < kPerVec; ++e) v[r][e] = qt[e];
+    } else {
+#pragma unroll
+      for (uint32_t e = 0; e < kPerVec; ++e) v[r][e] = i + e < count ? data[i + e] : T(0);
+    }
+  }
+#pragma unroll
+  for (uint32_t r = 0; r < kSmallRows; ++r) {
+    T sum = 0;
+#pragma unroll
+    for (uint32_t e = 0; e < kPerVec; ++e) sum += v[r][e];
+    const T inc = warp_inclusive_sum<T>(sum);
+    at[r] = run + inc - sum;
+    run += __shfl_sync(kFullMask, inc, kWarp - 1);
+  }
+  if (lane == 0) s_warp[warp] = run;
+  __syncthreads();
+  T before = 0;
+#pragma unroll
+  for (uint32_t w = 0; w < kWarps; ++w)
+    if (w < warp) before += s_warp[w];
+#pragma unroll
+  for (uint32_t r = 0; r < kSmallRows; ++r) {
+    const uint32_t i = first + r * kWarp * kPerVec;
+    T x = before + at[r];
+    uint4 q;
+    T *qt = reinterpret_cast<T *>(&q);
+#pragma unroll
+    for (uint32_t e = 0; e < kPerVec; ++e) {
+      const T y = x + v[r][e];
+      qt[e] = Inclusive ? y : x;
+      x = y;
+    }
+    if (Vectorised && i + kPerVec <= count) {
+      reinterpret_cast<uint4 *>(data)[i / kPerVec] = q;
+    } else {
+#pragma unroll
+      for (uint32_t e = 0; e < kPerVec; ++e)
+        if (i + e < count) data[i + e] = qt[e];
+    }
+  }
+}
+
 // Tiles for the element size and tile shape that need the most records (u64
 // in the smallest, 8 KB, tile).
 uint32_t max_tiles(uint32_t count) {
-  return ceil_div(count, TileShape<uint64_t, 64, 24>::kTile) + 1;
+  return ceil_div(count, Tile8<uint64_t>::kTile) + 1;
 }
 
+// Clears the header and the records of the call's tiles (at `base`, the
+// header's address) and launches the scan.
 template <class T, bool Inclusive, bool Vectorised, class S>
-void launch_shape(T *data, uint32_t count, const ScanLayout &ws,
-                  const typename RecordsFor<T>::type &records, cudaStream_t stream) {
+vx_status launch_shape(T *data, uint32_t count, const ScanLayout &ws, cudaStream_t stream) {
   const uint32_t tiles = ceil_div(count, S::kTile);
+  char *end = nullptr;
+  const auto records = make_records<T>(ws, tiles, &end);
+  char *base = reinterpret_cast<char *>(ws.tile_counter);
+  VX_TRY_CUDA(cudaMemsetAsync(base, 0, static_cast<size_t>(end - base), stream));
+  prof::Scope scope(sizeof(T) == 4 ? "scan_u32" : "scan_u64", stream);
   scan_kernel<T, Inclusive, Vectorised, S><<<tiles, S::kBlock, 0, stream>>>(data, count, ws,
                                                                             records);
+  return from_cuda(cudaGetLastError());
 }
 
-// Tile shape from the "scan.tile_kb" knob (32, 16 or 8 KB tiles).
+// One block when the data fits it; else the tile shape of the "scan.tile_kb"
+// knob (32, 16 or 8 KB tiles).
 template <class T, bool Inclusive, bool Vectorised>
-void launch_tuned(T *data, uint32_t count, const ScanLayout &ws,
-                  const typename RecordsFor<T>::type &records, cudaStream_t stream) {
+vx_status launch_tuned(T *data, uint32_t count, const ScanLayout &ws, cudaStream_t stream) {
+  if (count <= small_max<T>()) {
+    prof::Scope scope(sizeof(T) == 4 ? "scan_u32" : "scan_u64", stream);
+    scan_small_kernel<T, Inclusive, Vectorised><<<1, kSmallBlock, 0, stream>>>(data, count,
+                                                                               ws.status);
+    return from_cuda(cudaGetLastError());
+  }
   switch (tune::get(tune::kScanTileKb)) {
-  case 8:
-    launch_shape<T, Inclusive, Vectorised, TileShape<T, 64, 24>>(data, count, ws, records,
-                                                                 stream);
-    break;
-  case 16:
-    launch_shape<T, Inclusive, Vectorised, TileShape<T, 128, 12>>(data, count, ws, records,
-                                                                  stream);
-    break;
-  default:
-    launch_shape<T, Inclusive, Vectorised, TileShape<T>>(data, count, ws, records, stream);
+  case 8: return launch_shape<T, Inclusive, Vectorised, Tile8<T>>(data, count, ws, stream);
+  case 16: return launch_shape<T, Inclusive, Vectorised, Tile16<T>>(data, count, ws, stream);
+  default: return launch_shape<T, Inclusive, Vectorised, Tile32<T>>(data, count, ws, stream);
   }
 }
 
@@ -192,7 +286,7 @@ size_t workspace_size(uint32_t count) {
   return s.offset;
 }
 
-ScanLayout carve(void *workspace, uint32_t count, size_t elem_size) {
+ScanLayout carve(void *workspace, uint32_t count) {
   const uint32_t tiles = max_tiles(count);
   Carver c(workspace);
   ScanLayout l;
@@ -202,9 +296,6 @@ ScanLayout carve(void *workspace, uint32_t count, size_t elem_size) {
   l.rec_a = c.take<uint64_t>(tiles);
   l.rec_b = c.take<uint64_t>(tiles);
   l.rec_state = c.take<uint32_t>(tiles);
-  l.clear_bytes = elem_size == 4 ? (reinterpret_cast<char *>(l.rec_a + tiles) -
-                                    reinterpret_cast<char *>(hdr))
-                                 : c.offset;
   return l;
 }
 
@@ -215,23 +306,13 @@ vx_status scan_launch(T *data, uint32_t count, bool inclusive, void *workspace,
   if (count == 0) return VX_OK;
   if (workspace == nullptr || workspace_bytes < workspace_size(count))
     return VX_ERR_INVALID_VALUE;
-  const ScanLayout ws = carve(workspace, count, sizeof(T));
-  VX_TRY_CUDA(cudaMemsetAsync(workspace, 0, ws.clear_bytes, stream));
+  const ScanLayout ws = carve(workspace, count);
   const bool vec = (reinterpret_cast<uintptr_t>(data) & 15u) == 0;
-  const auto records = make_records<T>(ws);
-  prof::Scope scope(sizeof(T) == 4 ? "scan_u32" : "scan_u64", stream);
-  if (inclusive) {
-    if (vec)
-      launch_tuned<T, true, true>(data, count, ws, records, stream);
-    else
-      launch_tuned<T, true, false>(data, count, ws, records, stream);
-  } else {
-    if (vec)
-      launch_tuned<T, false, true>(data, count, ws, records, stream);
-    else
-      launch_tuned<T, false, false>(data, count, ws, records, stream);
-  }
-  return from_cuda(cudaGetLastError());
+  if (inclusive)
+    return vec ? launch_tuned<T, true, true>(data, count, ws, stream)
+               : launch_tuned<T, true, false>(data, count, ws, stream);
+  return vec ? launch_tuned<T, false, true>(data, count, ws, stream)
+             : launch_tuned<T, false, false>(data, count, ws, stream);
 }
 
 template vx_status scan_launch<uint32_t>(uint32_t *, uint32_t, bool, void *,
@@ -281,7 +362,7 @@ vx_status vx_scan_exclusive_sum_u64(uint64_t *data, uint32_t count,
 // or code that must not call cudaMalloc / cudaFree because those calls
 // synchronise the device.  This entry point takes no workspace: its look-back
 // scratch is one array in this library's own device memory, sized for at
-// most kNoAllocMaxCount elements (256 KiB plus a 256-byte header, held on
+// most kNoAllocMaxCount elements (272 KiB plus a 256-byte header, held on
 // every GPU that loads the library until the process exits).
 
 namespace vx::scan {
@@ -289,12 +370,14 @@ namespace {
 
 constexpr uint32_t kNoAllocMaxCount = 1u << 28;
 constexpr uint32_t kNoAllocTiles =
-    (kNoAllocMaxCount + TileShape<uint32_t>::kTile - 1) / TileShape<uint32_t>::kTile;
+    (kNoAllocMaxCount + Tile32<uint32_t>::kTile - 1) / Tile32<uint32_t>::kTile;
+constexpr uint32_t kNoAllocRecords = kNoAllocTiles + 2 * ((kNoAllocTiles + kGroup - 1) / kGroup);
 constexpr size_t kNoAllocHeader = 256; // tile counter, status word
 
-// [0, 256): tile counter and status; then one packed look-back record per tile.
+// [0, 256): tile counter and status; then a look-back record per tile and two
+// words per group of tiles.
 static __device__ __align__(256) unsigned char
-    g_noalloc_scratch[kNoAllocHeader + size_t(kNoAllocTiles) * sizeof(uint64_t)];
+    g_noalloc_scratch[kNoAllocHeader + size_t(kNoAllocRecords) * sizeof(uint64_t)];
 
 // Unique id of the calling thread's current CUDA context (0 when there is
 // none or the driver entry points are unavailable).  Context ids are never
@@ -371,21 +454,13 @@ vx_status vx_scan_exclusive_sum_u32_noalloc(uint32_t *data, uint32_t count,
   char *base = static_cast<char *>(noalloc_scratch(&err));
   if (base == nullptr) return vx::from_cuda(err);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  using S = TileShape<uint32_t>;
-  const uint32_t tiles = vx::ceil_div(count, S::kTile);
   ScanLayout ws{};
   ws.tile_counter = reinterpret_cast<uint32_t *>(base);
   ws.status = ws.tile_counter + 1;
   ws.rec_a = reinterpret_cast<uint64_t *>(base + kNoAllocHeader);
-  // The previous call's records are still there: clear the part this call uses.
-  VX_TRY_CUDA(cudaMemsetAsync(base, 0, kNoAllocHeader + size_t(tiles) * sizeof(uint64_t), s));
-  PackedRecords32 records{ws.rec_a};
-  vx::prof::Scope scope("scan_u32_noalloc", s);
   if ((reinterpret_cast<uintptr_t>(data) & 15u) == 0)
-    scan_kernel<uint32_t, false, true><<<tiles, S::kBlock, 0, s>>>(data, count, ws, records);
-  else
-    scan_kernel<uint32_t, false, false><<<tiles, S::kBlock, 0, s>>>(data, count, ws, records);
-  return vx::from_cuda(cudaGetLastError());
+    return launch_shape<uint32_t, false, true, Tile32<uint32_t>>(data, count, ws, s);
+  return launch_shape<uint32_t, false, false, Tile32<uint32_t>>(data, count, ws, s);
 }
 
 // Status of the most recent allocation-free scan on the current device:

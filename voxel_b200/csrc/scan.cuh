@@ -2,8 +2,9 @@
 // "Single-pass Parallel Prefix Scan with Decoupled Look-back"), written for
 // sm_100a: each tile arrives in shared memory by one bulk copy (TMA), a
 // dynamic tile id makes a tile only ever wait on tiles that are already
-// resident, a warp-parallel look-back reads 64 predecessors per round trip,
-// and a globaltimer bound limits every wait.
+// resident, a tile's 32-bit sum also goes into the sum of its group of 32
+// tiles, so that one round trip of three loads per lane reads 1,024
+// predecessors, and a globaltimer bound limits every wait.
 //
 // Replaces the reference's BlockBased<DecoupledLookback<WarpShuffleBlock<512,4>>>
 // (cuda/scan/block_based/decoupled_lookback.cuh:116-221), whose look-back is a
@@ -18,24 +19,69 @@ namespace vx::scan {
 // Look-back record states.
 constexpr uint32_t kNotReady = 0, kAggregate = 1, kInclusive = 2;
 
-// u32 sums pack state and value into one 64-bit word, so one relaxed load
-// observes both atomically.
-struct PackedRecords32 {
-  uint64_t *rec;
-  __device__ void publish(uint32_t tile, uint32_t state, uint32_t value) const {
-    st_relaxed_u64(rec + tile, (static_cast<uint64_t>(state) << 62) | value);
-  }
-  __device__ void read(int64_t tile, uint32_t &state, uint32_t &value) const {
-    if (tile < 0) {
-      state = kInclusive;
-      value = 0;
-      return;
-    }
-    const uint64_t r = ld_relaxed_u64(rec + tile);
-    state = static_cast<uint32_t>(r >> 62);
-    value = static_cast<uint32_t>(r);
-  }
+// u32 sums: a tile's record is its sum under a ready bit, one relaxed 64-bit
+// store.  The tile also adds its sum and 1 << kGroupCount to the word of its
+// group (32 tiles: the sums stay below the count), so a word whose count is 32
+// holds the whole group's sum; the group's last tile writes the group's
+// inclusive prefix, again under a ready bit.
+struct GroupRecords32 {
+  uint64_t *tile;
+  uint64_t *group_sum;
+  uint64_t *group_inc;
 };
+constexpr uint32_t kGroup = 32, kGroupCount = 40;
+constexpr uint64_t kReady = 1ull << 63;
+
+// Look-back for u32 sums, called by one full warp after lane 0 published the
+// tile (publish_group): lane l reads the record of its group's tile l and the
+// words of the l-th group back, until the tiles before it in its group and the
+// groups back to the nearest inclusive prefix are all there; a lane reads
+// again only what it has not got.  The smallest unfinished tile always finds
+// the inclusive prefix of the group before its own, so every tile ends.
+// Returns the sum of all earlier tiles (in every lane); on timeout sets
+// *status and returns a partial sum.
+__device__ __forceinline__ void publish_group(const GroupRecords32 &r, uint32_t tile,
+                                              uint32_t aggregate) {
+  atomicAdd(reinterpret_cast<unsigned long long *>(r.group_sum + tile / kGroup),
+            (1ull << kGroupCount) + aggregate);
+  st_relaxed_u64(r.tile + tile, kReady | aggregate);
+}
+
+__device__ __forceinline__ uint32_t group_lookback(const GroupRecords32 &r, uint32_t tile,
+                                                   uint32_t aggregate, uint32_t *status) {
+  const uint32_t lane = lane_id();
+  const uint32_t group = tile / kGroup, in = tile % kGroup;
+  const int64_t g = static_cast<int64_t>(group) - 1 - lane;
+  uint64_t own = lane < in ? 0ull : kReady;
+  uint64_t sum = 0, inc = g < 0 ? kReady : 0ull; // nothing before the first group
+  uint32_t exclusive = 0;
+  uint64_t t0 = 0;
+  for (;;) {
+    if (!(own & kReady)) own = ld_relaxed_u64(r.tile + group * kGroup + lane);
+    if (!(inc & kReady)) {
+      inc = ld_relaxed_u64(r.group_inc + g);
+      if ((sum >> kGroupCount) != kGroup) sum = ld_relaxed_u64(r.group_sum + g);
+    }
+    const bool own_all = __all_sync(kFullMask, (own & kReady) != 0);
+    const uint32_t found = __ballot_sync(kFullMask, (inc & kReady) != 0);
+    const uint32_t whole = __ballot_sync(kFullMask, (sum >> kGroupCount) == kGroup);
+    const uint32_t nearest = found ? __ffs(found) - 1u : 0u;
+    const uint32_t between = (1u << nearest) - 1u;
+    const bool there = own_all && found && (whole & between) == between;
+    if (there || (t0 != 0 && global_ns() - t0 > kWaitLimitNs)) {
+      if (!there && lane == 0) set_status(status, kDevTimeout);
+      uint32_t v = lane < in ? static_cast<uint32_t>(own) : 0u;
+      if (lane < nearest) v += static_cast<uint32_t>(sum);
+      else if (lane == nearest) v += static_cast<uint32_t>(inc);
+      exclusive = __reduce_add_sync(kFullMask, v);
+      break;
+    }
+    if (t0 == 0) t0 = global_ns();
+  }
+  if (in == kGroup - 1u && lane == 0)
+    st_relaxed_u64(r.group_inc + group, kReady | (exclusive + aggregate));
+  return exclusive;
+}
 
 // u64 sums keep the value beside a state word: value first, then a release
 // store of the state; readers acquire the state before reading the value.
@@ -60,11 +106,11 @@ struct SplitRecords64 {
 };
 
 template <class T> struct RecordsFor;
-template <> struct RecordsFor<uint32_t> { using type = PackedRecords32; };
+template <> struct RecordsFor<uint32_t> { using type = GroupRecords32; };
 template <> struct RecordsFor<uint64_t> { using type = SplitRecords64; };
 
-// Warp-parallel look-back, called by one full warp.  Publishes the tile's
-// aggregate, then reads the records of the previous 32 * R tiles at once
+// Warp-parallel look-back for u64 sums, called by one full warp after lane 0
+// published the tile's aggregate (publish_tile).  Reads the records of the previous 32 * R tiles at once
 // (lane l, row j reads distance l + 32 j: R coalesced loads in flight per
 // lane), accumulates back to the nearest inclusive record, publishes the
 // inclusive prefix and returns the exclusive prefix (valid in every lane).
@@ -76,11 +122,7 @@ template <class T, uint32_t R = 2, class Records>
 __device__ T warp_lookback(const Records &records, uint32_t tile, T aggregate,
                            uint32_t *status) {
   const uint32_t lane = lane_id();
-  if (tile == 0) {
-    if (lane == 0) records.publish(0, kInclusive, aggregate);
-    return T(0);
-  }
-  if (lane == 0) records.publish(tile, kAggregate, aggregate);
+  if (tile == 0) return T(0);
   T exclusive = 0;
   int64_t pos = static_cast<int64_t>(tile) - 1;
   const uint64_t t0 = global_ns();
@@ -131,34 +173,33 @@ __device__ T warp_lookback(const Records &records, uint32_t tile, T aggregate,
   return exclusive;
 }
 
-// Tile geometry: 256 threads x 8 rows of 16-byte vectors (a 32 KB tile);
-// row r of the tile is the contiguous range of kBlock vectors [r * kBlock,
-// (r + 1) * kBlock) and thread t owns vector t of every row.  The tile is
-// staged in shared memory by one bulk copy and scanned from there in two
-// passes, so a thread keeps only a few registers.  What bounds the bandwidth
-// is the bytes in flight per SM while tiles wait for their loads and
-// look-backs: registers would hold 128 KB of tiles per SM, shared memory
-// holds six 32 KB tiles.  Without the look-back this pipeline streams at
-// ~91 % of a device copy; the look-back chain (each tile waits for the
-// aggregates of all tiles before it) costs the rest.  Measured alternatives
-// on B200 (2^28 u32): 64 KB tiles x 3 per SM 0.63 ms, 128 KB x 1 0.72 ms,
-// 32 KB x 4 0.82 ms, this shape 0.61 ms; 512 threads x 4 rows held in
-// registers (2 per SM) 0.93 ms.
-// The "scan.tile_kb" knob offers two smaller tiles of the same 8 rows with
-// more of them resident (16 KB: 128 threads, 12 blocks / SM; 8 KB: 64
-// threads, 24 blocks / SM): about as many bytes staged per SM, but a tile
-// that waits for its predecessors' aggregates holds less of it.  On B200
-// they are slower (2^28 u32, median of 10: 32 KB 0.578 ms, 16 KB 0.598 ms,
-// 8 KB 0.672 ms; 2^27 u64: 0.755 / 0.815 / 0.924 ms): twice or four times
-// the tiles means as many more look-backs, each a round trip to L2.
-template <class T, uint32_t Block = 256, uint32_t MinBlocks = 6> struct TileShape {
+// Tile geometry: Block threads x Rows rows of 16-byte vectors, each warp a
+// contiguous part of the tile.  The tile is staged in shared memory by one
+// bulk copy and read from there twice (sums, then prefix sums), so a thread
+// keeps one value per row.  What bounds the bandwidth is the bytes in flight
+// per SM while tiles wait for their loads and for the tiles before them:
+// shared memory holds six 32 KB tiles.  On B200, 2^27 u32 (1.07 GB), 164 us at
+// the measured copy bandwidth:
+//   look-back over 64 tile records per round trip, rows scanned before the
+//     tile's sum is published (256 threads)                          301 us
+//   sum published first, rows scanned while the records are on the way 279 us
+//   group sums as above, 256 threads x 8 rows, 6 per SM              225 us
+//   the same, 128 threads x 16 rows, 6 per SM (this shape)       217-225 us
+//   48 KB tiles, 4 per SM 214 us; 64 KB, 3 per SM 223 us; 16 KB, 12 per SM
+//   250 us (more tiles: more round trips).
+// The "scan.tile_kb" knob offers 16 and 8 KB tiles.
+template <class T, uint32_t Block = 128, uint32_t Rows = 16, uint32_t MinBlocks = 6>
+struct TileShape {
   static constexpr uint32_t kBlock = Block;
-  static constexpr uint32_t kRows = 8;
+  static constexpr uint32_t kRows = Rows;
   static constexpr uint32_t kMinBlocks = MinBlocks;
   static constexpr uint32_t kPerVec = 16 / sizeof(T);
   static constexpr uint32_t kTile = kBlock * kRows * kPerVec;
   static constexpr uint32_t kWarps = kBlock / kWarp;
 };
+template <class T> using Tile32 = TileShape<T>;
+template <class T> using Tile16 = TileShape<T, 128, 8, 12>;
+template <class T> using Tile8 = TileShape<T, 64, 8, 24>;
 
 struct ScanLayout {
   uint32_t *tile_counter;
@@ -166,11 +207,10 @@ struct ScanLayout {
   uint64_t *rec_a;
   uint64_t *rec_b;
   uint32_t *rec_state;
-  size_t clear_bytes; // bytes from the workspace start to clear per call
 };
 
 size_t workspace_size(uint32_t count);
-ScanLayout carve(void *workspace, uint32_t count, size_t elem_size);
+ScanLayout carve(void *workspace, uint32_t count);
 
 template <class T>
 vx_status scan_launch(T *data, uint32_t count, bool inclusive, void *workspace,
