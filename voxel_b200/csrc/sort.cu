@@ -265,12 +265,16 @@ __global__ void __launch_bounds__(kBlock, (min_blocks<kItems, K>()))
   __shared__ uint32_t s_tile;
   // per (warp, digit): the warp's count, then its tile-local base
   __shared__ uint16_t s_warp_base[kWarps][kBins];
-  __shared__ uint32_t s_match[Ballots ? 1 : kWarps][Ballots ? 1 : kBins];
   __shared__ uint32_t s_count[Early ? kBins : 1];
   __shared__ uint32_t s_global[kBins];
   __shared__ uint32_t s_tmp[kWarps];
-  // The tile arrives here (input order), and later holds it sorted by digit.
-  __shared__ __align__(128) K s_keys[kTile];
+  // The tile arrives here (input order), and later holds it sorted by digit;
+  // in between, while the keys are in registers, the warps' match words (two
+  // per digit) lie in its place.
+  constexpr uint32_t kMatchBytes = Ballots ? 0u : 2u * kWarps * kBins * 4u;
+  constexpr uint32_t kKeySpace = kKeyBytes > kMatchBytes ? kKeyBytes : kMatchBytes;
+  __shared__ __align__(128) unsigned char s_key_space[kKeySpace];
+  K *const s_keys = reinterpret_cast<K *>(s_key_space);
   __shared__ __align__(128) uint32_t s_vals[HasValues ? kTile : 1];
 
   const uint32_t t = threadIdx.x, lane = lane_id(), warp = t / kWarp;
@@ -289,10 +293,6 @@ __global__ void __launch_bounds__(kBlock, (min_blocks<kItems, K>()))
   const uint32_t hist_t = pass_hist[t];
 #pragma unroll
   for (uint32_t w = 0; w < kWarps; ++w) s_warp_base[w][t] = 0;
-  if (!Ballots) {
-#pragma unroll
-    for (uint32_t w = 0; w < kWarps; ++w) s_match[w][t] = 0;
-  }
   if (Early) s_count[t] = 0;
   __syncthreads();
   const uint32_t tile = s_tile;
@@ -339,13 +339,12 @@ __global__ void __launch_bounds__(kBlock, (min_blocks<kItems, K>()))
 
   // Rank each key among the warp's earlier keys of its digit (stable: the
   // order of items, then of lanes).
+  if (Ballots) {
 #pragma unroll
-  for (uint32_t i = 0; i < kItems; ++i) {
-    const bool v = valid(i);
-    const uint32_t d = v ? digit_of(key[i], shift, mask) : kBins;
-    uint32_t peers;
-    if (Ballots) {
-      peers = kFullMask;
+    for (uint32_t i = 0; i < kItems; ++i) {
+      const bool v = valid(i);
+      const uint32_t d = v ? digit_of(key[i], shift, mask) : kBins;
+      uint32_t peers = kFullMask;
       if (!full) { // lanes without a key form their own group
         const uint32_t vb = __ballot_sync(kFullMask, v);
         peers = v ? vb : ~vb;
@@ -356,22 +355,56 @@ __global__ void __launch_bounds__(kBlock, (min_blocks<kItems, K>()))
         const uint32_t bb = __ballot_sync(kFullMask, bit);
         peers &= bit ? bb : ~bb;
       }
-    } else {
-      if (v) atomicOr(&s_match[warp][d], 1u << lane);
+      uint32_t pre = 0;
+      if (v) pre = s_warp_base[warp][d];
       __syncwarp();
-      peers = v ? s_match[warp][d] : 0u;
+      if (v && lane == 31u - __clz(peers)) // the digit's last lane
+        s_warp_base[warp][d] = static_cast<uint16_t>(pre + __popc(peers));
+      __syncwarp();
+      const uint32_t rk = pre + __popc(peers & lanemask_lt());
+      if (i & 1u) rank2[i / 2] |= rk << 16;
+      else rank2[i / 2] = rk;
     }
-    uint32_t pre = 0;
-    if (v) pre = s_warp_base[warp][d];
+  } else {
+    // Two items at a time, each with its own match words, so that the chain
+    // of shared-memory round trips (match, read back, count) runs half as
+    // often: the second item's keys also count the first's of their digit.
+    static_assert(kItems % 2 == 0, "items are ranked in pairs");
+    __syncthreads(); // every warp has its keys
+    uint32_t *const match0 = reinterpret_cast<uint32_t *>(s_key_space) + warp * 2u * kBins;
+    uint32_t *const match1 = match0 + kBins;
+#pragma unroll
+    for (uint32_t j = 0; j < 2u * kBins / (4u * kWarp); ++j)
+      reinterpret_cast<uint4 *>(match0)[j * kWarp + lane] = make_uint4(0u, 0u, 0u, 0u);
     __syncwarp();
-    if (v && lane == 31u - __clz(peers)) { // the digit's last lane
-      s_warp_base[warp][d] = static_cast<uint16_t>(pre + __popc(peers));
-      if (!Ballots) s_match[warp][d] = 0u;
+#pragma unroll
+    for (uint32_t i = 0; i < kItems; i += 2) {
+      const bool v0 = valid(i), v1 = valid(i + 1);
+      const uint32_t d0 = digit_of(key[i], shift, mask), d1 = digit_of(key[i + 1], shift, mask);
+      if (v0) atomicOr(&match0[d0], 1u << lane);
+      if (v1) atomicOr(&match1[d1], 1u << lane);
+      __syncwarp();
+      const uint32_t peers0 = match0[d0], also0 = match1[d0];
+      const uint32_t peers1 = match1[d1], also1 = match0[d1];
+      const uint32_t pre0 = s_warp_base[warp][d0];
+      const uint32_t pre1 = s_warp_base[warp][d1] + __popc(also1);
+      __syncwarp();
+      // One lane per digit adds both items' keys and clears its match words:
+      // the last lane of the second item, or of the first when the second has
+      // none of the digit.
+      if (v1 && lane == 31u - __clz(peers1)) {
+        s_warp_base[warp][d1] = static_cast<uint16_t>(pre1 + __popc(peers1));
+        match0[d1] = 0u;
+        match1[d1] = 0u;
+      }
+      if (v0 && also0 == 0u && lane == 31u - __clz(peers0)) {
+        s_warp_base[warp][d0] = static_cast<uint16_t>(pre0 + __popc(peers0));
+        match0[d0] = 0u;
+      }
+      __syncwarp();
+      rank2[i / 2] =
+          (pre0 + __popc(peers0 & lanemask_lt())) | ((pre1 + __popc(peers1 & lanemask_lt())) << 16);
     }
-    __syncwarp();
-    const uint32_t rk = pre + __popc(peers & lanemask_lt());
-    if (i & 1u) rank2[i / 2] |= rk << 16;
-    else rank2[i / 2] = rk;
   }
   __syncthreads();
 
@@ -393,11 +426,10 @@ __global__ void __launch_bounds__(kBlock, (min_blocks<kItems, K>()))
     }
   }
   const uint32_t global_start = block_exclusive_256(hist_t, s_tmp);
-  const uint32_t exclusive = digit_lookback(records, tile, t, tile_count, status);
-  s_global[t] = global_start + exclusive - digit_off;
-  __syncthreads();
 
-  // Sort the tile in shared memory (its input copy is in registers now).
+  // Sort the tile in shared memory (its input copy is in registers now; the
+  // bases are complete after the block scan's barriers), while the tiles
+  // before this one publish their counts.
 #pragma unroll
   for (uint32_t i = 0; i < kItems; ++i) {
     if (!valid(i)) continue;
@@ -407,6 +439,8 @@ __global__ void __launch_bounds__(kBlock, (min_blocks<kItems, K>()))
     s_keys[pos] = key[i];
     if (HasValues) s_vals[pos] = val[i];
   }
+  const uint32_t exclusive = digit_lookback(records, tile, t, tile_count, status);
+  s_global[t] = global_start + exclusive - digit_off;
   __syncthreads();
 
   // Write the tile's runs out in order: consecutive threads, consecutive
