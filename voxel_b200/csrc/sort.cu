@@ -54,7 +54,7 @@ template <> struct Shape<uint64_t> {
   static constexpr uint32_t kSmall = 8, kLarge = 10;
 };
 template <uint32_t Items, class K> constexpr uint32_t min_blocks() {
-  return Items == Shape<K>::kSmall ? 4u : 3u;
+  return Items == Shape<K>::kSmall ? 5u : 4u;
 }
 // Tiles of the small setting: the most tiles, so the workspace covers both.
 template <class K> inline uint32_t max_tiles(uint32_t count) {
@@ -235,6 +235,23 @@ __device__ __forceinline__ uint32_t digit_lookback(uint32_t *records, uint32_t t
   return exclusive;
 }
 
+// A block's shared memory, above the 48 KB that a kernel may declare.
+template <class K, bool HasValues, uint32_t kItems, bool Early, bool Ballots>
+struct PartitionSmem {
+  static constexpr uint32_t kTile = kBlock * kItems;
+  // The tile arrives here (input order), and later lies here sorted by digit.
+  alignas(128) K keys[kTile];
+  alignas(128) uint32_t vals[HasValues ? kTile : 1];
+  alignas(16) uint32_t match[Ballots ? 1 : kWarps][2][Ballots ? 1 : kBins];
+  // per (warp, digit): the warp's count, then its tile-local base
+  uint16_t warp_base[kWarps][kBins];
+  uint32_t global[kBins];
+  uint32_t count[Early ? kBins : 1];
+  uint32_t tmp[kWarps];
+  uint64_t bar;
+  uint32_t tile;
+};
+
 // Early = publish the tile's digit counts (from a shared-atomic histogram)
 // before ranking, so later tiles' look-backs wait less; otherwise they are
 // published after ranking, from the per-warp counts.
@@ -257,53 +274,47 @@ __global__ void __launch_bounds__(kBlock, (min_blocks<kItems, K>()))
                      const uint32_t *__restrict__ pass_hist,
                      uint32_t *records, uint32_t *tile_counter,
                      uint32_t *status, bool aligned) {
-  constexpr uint32_t kTile = kBlock * kItems;
+  using Smem = PartitionSmem<K, HasValues, kItems, Early, Ballots>;
+  constexpr uint32_t kTile = Smem::kTile;
   constexpr uint32_t kKeyBytes = kTile * sizeof(K);
   constexpr uint32_t kValBytes = HasValues ? kTile * 4u : 0u;
   static_assert(kTile <= 0xffffu, "ranks are 16-bit");
-  __shared__ uint64_t s_bar;
-  __shared__ uint32_t s_tile;
-  // per (warp, digit): the warp's count, then its tile-local base
-  __shared__ uint16_t s_warp_base[kWarps][kBins];
-  __shared__ uint32_t s_count[Early ? kBins : 1];
-  __shared__ uint32_t s_global[kBins];
-  __shared__ uint32_t s_tmp[kWarps];
-  // The tile arrives here (input order), and later holds it sorted by digit;
-  // in between, while the keys are in registers, the warps' match words (two
-  // per digit) lie in its place.
-  constexpr uint32_t kMatchBytes = Ballots ? 0u : 2u * kWarps * kBins * 4u;
-  constexpr uint32_t kKeySpace = kKeyBytes > kMatchBytes ? kKeyBytes : kMatchBytes;
-  __shared__ __align__(128) unsigned char s_key_space[kKeySpace];
-  K *const s_keys = reinterpret_cast<K *>(s_key_space);
-  __shared__ __align__(128) uint32_t s_vals[HasValues ? kTile : 1];
+  extern __shared__ __align__(128) unsigned char s_raw[];
+  Smem &s = *reinterpret_cast<Smem *>(s_raw);
+  K *const s_keys = s.keys;
+  uint32_t *const s_vals = s.vals;
 
   const uint32_t t = threadIdx.x, lane = lane_id(), warp = t / kWarp;
   if (t == 0) {
     const uint32_t tile = atomicAdd(tile_counter, 1u);
-    s_tile = tile;
+    s.tile = tile;
     if (aligned && static_cast<uint64_t>(tile + 1) * kTile <= count) {
       const uint64_t b = static_cast<uint64_t>(tile) * kTile;
-      mbar_init(&s_bar, 1);
-      mbar_arrive_expect_tx(&s_bar, kKeyBytes + kValBytes);
-      bulk_load(s_keys, in_keys + b, kKeyBytes, &s_bar);
-      if (HasValues) bulk_load(s_vals, in_vals + b, kValBytes, &s_bar);
+      mbar_init(&s.bar, 1);
+      mbar_arrive_expect_tx(&s.bar, kKeyBytes + kValBytes);
+      bulk_load(s_keys, in_keys + b, kKeyBytes, &s.bar);
+      if (HasValues) bulk_load(s_vals, in_vals + b, kValBytes, &s.bar);
     }
   }
   // Where each digit's run of this pass starts (independent of the tile).
   const uint32_t hist_t = pass_hist[t];
 #pragma unroll
-  for (uint32_t w = 0; w < kWarps; ++w) s_warp_base[w][t] = 0;
-  if (Early) s_count[t] = 0;
+  for (uint32_t w = 0; w < kWarps; ++w) s.warp_base[w][t] = 0;
+  if (!Ballots) {
+#pragma unroll
+    for (uint32_t w = 0; w < kWarps; ++w) s.match[w][0][t] = s.match[w][1][t] = 0;
+  }
+  if (Early) s.count[t] = 0;
   __syncthreads();
-  const uint32_t tile = s_tile;
+  const uint32_t tile = s.tile;
   const uint32_t tile_base = tile * kTile; // count < 2^30
   const uint32_t valid_in_tile = count - tile_base < kTile ? count - tile_base : kTile;
   const bool full = valid_in_tile == kTile;
   if (aligned && full) {
-    if (!mbar_wait(&s_bar, 0)) {
+    if (!mbar_wait(&s.bar, 0)) {
       // Never expected: report, let the copies land, give up on this tile.
       if (t == 0) set_status(status, kDevTimeout);
-      mbar_wait(&s_bar, 0);
+      mbar_wait(&s.bar, 0);
       return;
     }
   } else {
@@ -318,23 +329,26 @@ __global__ void __launch_bounds__(kBlock, (min_blocks<kItems, K>()))
   // past the end of a partial tile holds no key (digit kBins).
   auto valid = [&](uint32_t i) { return full || warp_first + i * kWarp + lane < valid_in_tile; };
 
-  K key[kItems];
-  uint32_t val[kItems];
-  uint32_t rank2[(kItems + 1) / 2]; // ranks within the warp's keys of a digit, 16 bits each
+  // The digits of the lane's keys, four to a register; the keys themselves
+  // stay in shared memory while they are ranked, so that four blocks' worth
+  // of registers is enough.
+  uint32_t digits[(kItems + 3) / 4];
 #pragma unroll
   for (uint32_t i = 0; i < kItems; ++i) {
-    const uint32_t j = warp_first + i * kWarp + lane;
-    key[i] = valid(i) ? s_keys[j] : K(0);
-    val[i] = HasValues && valid(i) ? s_vals[j] : 0u;
+    const uint32_t d =
+        valid(i) ? digit_of(s_keys[warp_first + i * kWarp + lane], shift, mask) : 0u;
+    digits[i / 4] = (i % 4 ? digits[i / 4] : 0u) | (d << (8 * (i % 4)));
   }
+  auto digit = [&](uint32_t i) { return (digits[i / 4] >> (8 * (i % 4))) & 0xffu; };
+  uint32_t rank2[(kItems + 1) / 2]; // ranks within the warp's keys of a digit, 16 bits each
 
   uint32_t *rec = records + static_cast<size_t>(tile) * kBins + t;
   if (Early) {
 #pragma unroll
     for (uint32_t i = 0; i < kItems; ++i)
-      if (valid(i)) atomicAdd(&s_count[digit_of(key[i], shift, mask)], 1u);
+      if (valid(i)) atomicAdd(&s.count[digit(i)], 1u);
     __syncthreads();
-    st_relaxed_u32(rec, (tile == 0 ? kRecInc : kRecAgg) | s_count[t]);
+    st_relaxed_u32(rec, (tile == 0 ? kRecInc : kRecAgg) | s.count[t]);
   }
 
   // Rank each key among the warp's earlier keys of its digit (stable: the
@@ -343,7 +357,7 @@ __global__ void __launch_bounds__(kBlock, (min_blocks<kItems, K>()))
 #pragma unroll
     for (uint32_t i = 0; i < kItems; ++i) {
       const bool v = valid(i);
-      const uint32_t d = v ? digit_of(key[i], shift, mask) : kBins;
+      const uint32_t d = v ? digit(i) : kBins;
       uint32_t peers = kFullMask;
       if (!full) { // lanes without a key form their own group
         const uint32_t vb = __ballot_sync(kFullMask, v);
@@ -356,10 +370,10 @@ __global__ void __launch_bounds__(kBlock, (min_blocks<kItems, K>()))
         peers &= bit ? bb : ~bb;
       }
       uint32_t pre = 0;
-      if (v) pre = s_warp_base[warp][d];
+      if (v) pre = s.warp_base[warp][d];
       __syncwarp();
       if (v && lane == 31u - __clz(peers)) // the digit's last lane
-        s_warp_base[warp][d] = static_cast<uint16_t>(pre + __popc(peers));
+        s.warp_base[warp][d] = static_cast<uint16_t>(pre + __popc(peers));
       __syncwarp();
       const uint32_t rk = pre + __popc(peers & lanemask_lt());
       if (i & 1u) rank2[i / 2] |= rk << 16;
@@ -370,35 +384,29 @@ __global__ void __launch_bounds__(kBlock, (min_blocks<kItems, K>()))
     // of shared-memory round trips (match, read back, count) runs half as
     // often: the second item's keys also count the first's of their digit.
     static_assert(kItems % 2 == 0, "items are ranked in pairs");
-    __syncthreads(); // every warp has its keys
-    uint32_t *const match0 = reinterpret_cast<uint32_t *>(s_key_space) + warp * 2u * kBins;
-    uint32_t *const match1 = match0 + kBins;
-#pragma unroll
-    for (uint32_t j = 0; j < 2u * kBins / (4u * kWarp); ++j)
-      reinterpret_cast<uint4 *>(match0)[j * kWarp + lane] = make_uint4(0u, 0u, 0u, 0u);
-    __syncwarp();
+    uint32_t *const match0 = s.match[warp][0], *const match1 = s.match[warp][1];
 #pragma unroll
     for (uint32_t i = 0; i < kItems; i += 2) {
       const bool v0 = valid(i), v1 = valid(i + 1);
-      const uint32_t d0 = digit_of(key[i], shift, mask), d1 = digit_of(key[i + 1], shift, mask);
+      const uint32_t d0 = digit(i), d1 = digit(i + 1);
       if (v0) atomicOr(&match0[d0], 1u << lane);
       if (v1) atomicOr(&match1[d1], 1u << lane);
       __syncwarp();
       const uint32_t peers0 = match0[d0], also0 = match1[d0];
       const uint32_t peers1 = match1[d1], also1 = match0[d1];
-      const uint32_t pre0 = s_warp_base[warp][d0];
-      const uint32_t pre1 = s_warp_base[warp][d1] + __popc(also1);
+      const uint32_t pre0 = s.warp_base[warp][d0];
+      const uint32_t pre1 = s.warp_base[warp][d1] + __popc(also1);
       __syncwarp();
       // One lane per digit adds both items' keys and clears its match words:
       // the last lane of the second item, or of the first when the second has
       // none of the digit.
       if (v1 && lane == 31u - __clz(peers1)) {
-        s_warp_base[warp][d1] = static_cast<uint16_t>(pre1 + __popc(peers1));
+        s.warp_base[warp][d1] = static_cast<uint16_t>(pre1 + __popc(peers1));
         match0[d1] = 0u;
         match1[d1] = 0u;
       }
       if (v0 && also0 == 0u && lane == 31u - __clz(peers0)) {
-        s_warp_base[warp][d0] = static_cast<uint16_t>(pre0 + __popc(peers0));
+        s.warp_base[warp][d0] = static_cast<uint16_t>(pre0 + __popc(peers0));
         match0[d0] = 0u;
       }
       __syncwarp();
@@ -412,35 +420,45 @@ __global__ void __launch_bounds__(kBlock, (min_blocks<kItems, K>()))
   uint32_t wc[kWarps], tile_count = 0;
 #pragma unroll
   for (uint32_t w = 0; w < kWarps; ++w) {
-    wc[w] = s_warp_base[w][t];
+    wc[w] = s.warp_base[w][t];
     tile_count += wc[w];
   }
   if (!Early) st_relaxed_u32(rec, (tile == 0 ? kRecInc : kRecAgg) | tile_count);
-  const uint32_t digit_off = block_exclusive_256(tile_count, s_tmp);
+  const uint32_t digit_off = block_exclusive_256(tile_count, s.tmp);
   {
     uint32_t run = digit_off;
 #pragma unroll
     for (uint32_t w = 0; w < kWarps; ++w) {
-      s_warp_base[w][t] = static_cast<uint16_t>(run);
+      s.warp_base[w][t] = static_cast<uint16_t>(run);
       run += wc[w];
     }
   }
-  const uint32_t global_start = block_exclusive_256(hist_t, s_tmp);
+  const uint32_t global_start = block_exclusive_256(hist_t, s.tmp);
 
-  // Sort the tile in shared memory (its input copy is in registers now; the
-  // bases are complete after the block scan's barriers), while the tiles
-  // before this one publish their counts.
+  // Sort the tile in shared memory, through registers (the bases are complete
+  // after the block scan's barriers), while the tiles before this one publish
+  // their counts.
+  {
+    K key[kItems];
+    uint32_t val[HasValues ? kItems : 1];
 #pragma unroll
-  for (uint32_t i = 0; i < kItems; ++i) {
-    if (!valid(i)) continue;
-    const uint32_t d = digit_of(key[i], shift, mask);
-    const uint32_t rk = (i & 1u) ? (rank2[i / 2] >> 16) : (rank2[i / 2] & 0xffffu);
-    const uint32_t pos = s_warp_base[warp][d] + rk;
-    s_keys[pos] = key[i];
-    if (HasValues) s_vals[pos] = val[i];
+    for (uint32_t i = 0; i < kItems; ++i) {
+      const uint32_t j = warp_first + i * kWarp + lane;
+      key[i] = valid(i) ? s_keys[j] : K(0);
+      if (HasValues) val[i] = valid(i) ? s_vals[j] : 0u;
+    }
+    __syncthreads(); // every key is in a register
+#pragma unroll
+    for (uint32_t i = 0; i < kItems; ++i) {
+      if (!valid(i)) continue;
+      const uint32_t rk = (i & 1u) ? (rank2[i / 2] >> 16) : (rank2[i / 2] & 0xffffu);
+      const uint32_t pos = s.warp_base[warp][digit(i)] + rk;
+      s_keys[pos] = key[i];
+      if (HasValues) s_vals[pos] = val[i];
+    }
   }
   const uint32_t exclusive = digit_lookback(records, tile, t, tile_count, status);
-  s_global[t] = global_start + exclusive - digit_off;
+  s.global[t] = global_start + exclusive - digit_off;
   __syncthreads();
 
   // Write the tile's runs out in order: consecutive threads, consecutive
@@ -451,7 +469,7 @@ __global__ void __launch_bounds__(kBlock, (min_blocks<kItems, K>()))
     const uint32_t j = r * kBlock + t;
     if (!full && j >= valid_in_tile) break;
     const K k = s_keys[j];
-    const uint32_t dst = s_global[digit_of(k, shift, mask)] + j;
+    const uint32_t dst = s.global[digit_of(k, shift, mask)] + j;
     out_keys[dst] = k;
     if (HasValues) out_vals[dst] = s_vals[j];
   }
@@ -501,29 +519,32 @@ vx_status sort_pairs(K *keys, uint32_t *values, uint32_t count,
     uint32_t *rec = l.records + static_cast<size_t>(p) * tiles * kBins;
     prof::Scope scope(sizeof(K) == 4 ? "sort_partition_u32" : "sort_partition_u64", stream);
     const bool aligned = aligned16(src_k) && (values == nullptr || aligned16(src_v));
-    auto launch = [&](auto kernel) {
-      kernel<<<tiles, kBlock, 0, stream>>>(src_k, src_v, dst_k, dst_v, count, info.shift[p],
-                                           info.mask[p], l.hist + p * kBins, rec,
-                                           l.counters + 2 + p, l.counters + 1, aligned);
+    auto launch = [&](auto kernel, size_t smem) {
+      const cudaError_t e = cudaFuncSetAttribute(
+          kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+      if (e != cudaSuccess) return e;
+      kernel<<<tiles, kBlock, smem, stream>>>(src_k, src_v, dst_k, dst_v, count, info.shift[p],
+                                              info.mask[p], l.hist + p * kBins, rec,
+                                              l.counters + 2 + p, l.counters + 1, aligned);
+      return cudaGetLastError();
     };
     // (values, items, early, ballots) -> one of 16 instantiations
     auto by_ballots = [&](auto hv, auto it, auto ea) {
       constexpr bool HV = decltype(hv)::value, E = decltype(ea)::value;
       constexpr uint32_t I = decltype(it)::value;
-      if (ballots) launch(partition_kernel<K, HV, I, E, true>);
-      else launch(partition_kernel<K, HV, I, E, false>);
+      return ballots ? launch(partition_kernel<K, HV, I, E, true>,
+                              sizeof(PartitionSmem<K, HV, I, E, true>))
+                     : launch(partition_kernel<K, HV, I, E, false>,
+                              sizeof(PartitionSmem<K, HV, I, E, false>));
     };
     auto by_early = [&](auto hv, auto it) {
-      if (early) by_ballots(hv, it, std::true_type{});
-      else by_ballots(hv, it, std::false_type{});
+      return early ? by_ballots(hv, it, std::true_type{}) : by_ballots(hv, it, std::false_type{});
     };
     auto by_items = [&](auto hv) {
-      if (large) by_early(hv, std::integral_constant<uint32_t, Shape<K>::kLarge>{});
-      else by_early(hv, std::integral_constant<uint32_t, Shape<K>::kSmall>{});
+      return large ? by_early(hv, std::integral_constant<uint32_t, Shape<K>::kLarge>{})
+                   : by_early(hv, std::integral_constant<uint32_t, Shape<K>::kSmall>{});
     };
-    if (values != nullptr) by_items(std::true_type{});
-    else by_items(std::false_type{});
-    VX_TRY_CUDA(cudaGetLastError());
+    VX_TRY_CUDA(values != nullptr ? by_items(std::true_type{}) : by_items(std::false_type{}));
     std::swap(src_k, dst_k);
     std::swap(src_v, dst_v);
   }
