@@ -10,12 +10,13 @@
 //          (TMA); each warp takes 32 x kItems of them and ranks them by digit
 //          with __match_any_sync (stable: rank follows the original order
 //          inside the warp);
-//        - warp counts are combined per digit, the tile publishes its digit
-//          counts and looks back over predecessor tiles per digit, eight
-//          tiles per round trip (bounded by the GPU timer);
-//        - keys and payloads are first sorted inside the tile in shared
-//          memory, then written out in that order so consecutive threads write
-//          consecutive addresses of each digit's run.
+//        - warp counts are combined per digit and the tile publishes its digit
+//          counts, also into the sums of its group of 8 and of 64 tiles;
+//        - keys and payloads are sorted inside the tile in shared memory;
+//        - it looks back over the tiles, groups and super-groups before it per
+//          digit (bounded by the GPU timer) and writes the tile out in its
+//          sorted order, so consecutive threads write consecutive addresses
+//          of each digit's run.
 //
 // Replaces algo::cuda::sort::sort_by_key with OneSweepPass
 // (cuda/sort/radix/onesweep/host.cuh:135-204, partition.cuh:117-200,
@@ -37,9 +38,29 @@ constexpr uint32_t kWarps = kBlock / kWarp;
 constexpr uint32_t kMaxPasses = 8;
 constexpr uint32_t kMaxCount = (1u << 30) - 1u;
 
-// Look-back record: state in bits 30-31, count in bits 0-29.
-constexpr uint32_t kRecAgg = 1u << 30, kRecInc = 2u << 30;
-constexpr uint32_t kRecValue = (1u << 30) - 1u;
+// Look-back words, one per digit each (the block's threads are the digits):
+//   per tile: its count under a ready bit;
+//   per group of 8 tiles and per super-group of 64: the sum of the counts
+//     plus the number of tiles << 24 (64 tiles of 4,096 keys sum below 2^24);
+//   per super-group: the inclusive count over all tiles up to its last one,
+//     under a ready bit.
+constexpr uint32_t kReady = 1u << 31;
+constexpr uint32_t kGroup = 8, kSuper = 64, kTiles = 24;
+constexpr uint32_t kSumMask = (1u << kTiles) - 1u;
+struct Records {
+  uint32_t *tile, *group, *super, *inclusive; // [...][256]
+};
+inline uint32_t record_rows(uint32_t tiles) {
+  return tiles + ceil_div(tiles, kGroup) + 2u * ceil_div(tiles, kSuper);
+}
+inline Records records_of(uint32_t *words, uint32_t tiles) {
+  Records r;
+  r.tile = words;
+  r.group = r.tile + static_cast<size_t>(tiles) * 256u;
+  r.super = r.group + static_cast<size_t>(ceil_div(tiles, kGroup)) * 256u;
+  r.inclusive = r.super + static_cast<size_t>(ceil_div(tiles, kSuper)) * 256u;
+  return r;
+}
 
 // Items per thread of the partition kernel (the tile is 256 x items keys):
 // the small setting fits four blocks per SM (64 registers, ~35 KB of shared
@@ -92,10 +113,9 @@ struct PassInfo {
 struct Layout {
   uint32_t *counters;  // [1] device status, [2 + p] tile counter of pass p
   uint32_t *hist;      // passes x 256 digit counts
-  uint32_t *records;   // passes x tiles x 256
+  uint32_t *records;   // passes x record_rows(tiles) x 256
   void *tmp_keys;
   uint32_t *tmp_vals;
-  size_t clear_bytes;
 };
 
 template <class K> Layout carve(void *ws, uint32_t count, uint32_t passes) {
@@ -104,8 +124,7 @@ template <class K> Layout carve(void *ws, uint32_t count, uint32_t passes) {
   Layout l;
   l.counters = c.take<uint32_t>(kMaxPasses + 2);
   l.hist = c.take<uint32_t>(kMaxPasses * kBins);
-  l.records = c.take<uint32_t>(static_cast<size_t>(passes) * tiles * kBins);
-  l.clear_bytes = c.offset;
+  l.records = c.take<uint32_t>(static_cast<size_t>(passes) * record_rows(tiles) * kBins);
   l.tmp_keys = c.take<K>(count);
   l.tmp_vals = c.take<uint32_t>(count);
   return l;
@@ -116,7 +135,7 @@ template <class K> size_t workspace_bytes(uint32_t count, uint32_t passes) {
   Sizer s;
   s.take<uint32_t>(kMaxPasses + 2);
   s.take<uint32_t>(kMaxPasses * kBins);
-  s.take<uint32_t>(static_cast<size_t>(passes) * tiles * kBins);
+  s.take<uint32_t>(static_cast<size_t>(passes) * record_rows(tiles) * kBins);
   s.take<K>(count);
   s.take<uint32_t>(count);
   return s.offset;
@@ -184,54 +203,99 @@ __device__ __forceinline__ uint32_t block_exclusive_256(uint32_t v,
   return r;
 }
 
-// Per-digit decoupled look-back over predecessor tiles, once this tile's
-// count is published: thread t (digit t) reads the records of kWindow
-// predecessors at once (independent loads, one round trip to L2), sums back
-// to the nearest inclusive record and retries the window while a tile before
-// that one has not published its count (bounded by the GPU timer); then it
-// publishes this tile's inclusive count.  Returns the digit's count over all
-// earlier tiles.
-__device__ __forceinline__ uint32_t digit_lookback(uint32_t *records, uint32_t tile, uint32_t t,
-                                                   uint32_t tile_count, uint32_t *status) {
-  if (tile == 0) return 0;
-  constexpr uint32_t kWindow = 8;
-  uint32_t exclusive = 0;
+// Thread t publishes the tile's count of digit t.
+__device__ __forceinline__ void publish_count(const Records &r, uint32_t tile, uint32_t t,
+                                              uint32_t count) {
+  st_relaxed_u32(r.tile + static_cast<size_t>(tile) * kBins + t, kReady | count);
+  atomicAdd(r.group + static_cast<size_t>(tile / kGroup) * kBins + t, (1u << kTiles) | count);
+  atomicAdd(r.super + static_cast<size_t>(tile / kSuper) * kBins + t, (1u << kTiles) | count);
+}
+
+// Reads *p until ready(value) (bounded by the GPU timer); `v` is the value
+// read already.
+template <class Ready>
+__device__ __forceinline__ uint32_t wait_word(const uint32_t *p, uint32_t v, Ready ready,
+                                              uint32_t *status) {
+  if (ready(v)) return v;
   const uint64_t t0 = global_ns();
-  int64_t pred = static_cast<int64_t>(tile) - 1;
   for (;;) {
-    uint32_t r[kWindow];
-#pragma unroll
-    for (uint32_t j = 0; j < kWindow; ++j)
-      r[j] = pred - static_cast<int64_t>(j) >= 0
-                 ? ld_relaxed_u32(records + static_cast<size_t>(pred - j) * kBins + t)
-                 : kRecInc;
-    uint32_t sum = 0;
-    bool found = false, wait = false;
-#pragma unroll
-    for (uint32_t j = 0; j < kWindow; ++j) {
-      if (found || wait) continue;
-      const uint32_t state = r[j] & ~kRecValue;
-      if (state == 0) {
-        wait = true;
-      } else {
-        sum += r[j] & kRecValue;
-        found = state == kRecInc;
-      }
+    __nanosleep(20);
+    v = ld_relaxed_u32(p);
+    if (ready(v)) return v;
+    if (global_ns() - t0 > kWaitLimitNs) {
+      set_status(status, kDevTimeout);
+      return 0;
     }
-    if (wait) {
-      if (global_ns() - t0 > kWaitLimitNs) {
-        set_status(status, kDevTimeout);
-        break;
-      }
-      __nanosleep(20);
-      continue;
-    }
-    exclusive += sum;
-    if (found) break;
-    pred -= kWindow;
   }
-  st_relaxed_u32(records + static_cast<size_t>(tile) * kBins + t,
-                 kRecInc | (exclusive + tile_count));
+}
+
+// Per-digit look-back, once every tile publishes with publish_count: the sum
+// of the tiles before this one in its group, of the groups before it in its
+// super-group, and of the super-groups back to the nearest inclusive count
+// (the last tile of a super-group publishes that one, so the smallest
+// unfinished tile always finds its predecessor's).  The words of the first
+// round are read together; afterwards only a word that is not there yet is
+// read again.  Reading eight tiles a round trip back to an inclusive one took
+// a dozen rounds with ~600 tiles in flight, ~100 of a pass's 169 instructions
+// per u64 key.  Returns the digit's count over all earlier tiles.
+__device__ __forceinline__ uint32_t digit_lookback(const Records &r, uint32_t tile, uint32_t t,
+                                                   uint32_t tile_count, uint32_t *status) {
+  constexpr uint32_t kFirst = 4; // super-groups read in the first round
+  const uint32_t in = tile % kGroup, group = tile / kGroup, gin = group % (kSuper / kGroup);
+  const uint32_t super = tile / kSuper;
+  const uint32_t *tiles = r.tile + static_cast<size_t>(tile - in) * kBins + t;
+  const uint32_t *groups = r.group + static_cast<size_t>(group - gin) * kBins + t;
+  auto row = [&](const uint32_t *words, uint32_t i) {
+    return words + static_cast<size_t>(i) * kBins + t;
+  };
+  uint32_t own[kGroup - 1], grp[kSuper / kGroup - 1], sum[kFirst], inc[kFirst];
+#pragma unroll
+  for (uint32_t j = 0; j < kGroup - 1; ++j) own[j] = j < in ? ld_relaxed_u32(tiles + j * kBins) : 0u;
+#pragma unroll
+  for (uint32_t j = 0; j < kSuper / kGroup - 1; ++j)
+    grp[j] = j < gin ? ld_relaxed_u32(groups + j * kBins) : 0u;
+#pragma unroll
+  for (uint32_t j = 0; j < kFirst; ++j) {
+    inc[j] = super > j ? ld_relaxed_u32(row(r.inclusive, super - 1 - j)) : 0u;
+    sum[j] = super > j ? ld_relaxed_u32(row(r.super, super - 1 - j)) : 0u;
+  }
+  auto tile_ready = [](uint32_t v) { return (v & kReady) != 0; };
+  auto group_ready = [](uint32_t v) { return (v >> kTiles) == kGroup; };
+  auto super_ready = [](uint32_t v) { return (v >> kTiles) == kSuper; };
+  uint32_t exclusive = 0;
+  bool found = super == 0;
+#pragma unroll
+  for (uint32_t j = 0; j < kFirst; ++j) {
+    if (found || super <= j) continue;
+    if (inc[j] & kReady) {
+      exclusive += inc[j] & ~kReady;
+      found = true;
+    } else {
+      exclusive += wait_word(row(r.super, super - 1 - j), sum[j], super_ready, status) & kSumMask;
+      found = super == j + 1; // the first super-group: nothing before it
+    }
+  }
+  for (uint32_t k = super - 1 - kFirst; !found; --k) { // (super > kFirst here)
+    const uint32_t v = ld_relaxed_u32(row(r.inclusive, k));
+    const uint32_t w = ld_relaxed_u32(row(r.super, k));
+    if (v & kReady) {
+      exclusive += v & ~kReady;
+      found = true;
+    } else {
+      exclusive += wait_word(row(r.super, k), w, super_ready, status) & kSumMask;
+      found = k == 0;
+    }
+  }
+#pragma unroll
+  for (uint32_t j = 0; j < kSuper / kGroup - 1; ++j)
+    if (j < gin)
+      exclusive += wait_word(groups + j * kBins, grp[j], group_ready, status) & kSumMask;
+#pragma unroll
+  for (uint32_t j = 0; j < kGroup - 1; ++j)
+    if (j < in) exclusive += wait_word(tiles + j * kBins, own[j], tile_ready, status) & ~kReady;
+  if (tile % kSuper == kSuper - 1)
+    st_relaxed_u32(r.inclusive + static_cast<size_t>(super) * kBins + t,
+                   kReady | (exclusive + tile_count));
   return exclusive;
 }
 
@@ -272,7 +336,7 @@ __global__ void __launch_bounds__(kBlock, (min_blocks<kItems, K>()))
                      K *__restrict__ out_keys, uint32_t *__restrict__ out_vals,
                      uint32_t count, uint32_t shift, uint32_t mask,
                      const uint32_t *__restrict__ pass_hist,
-                     uint32_t *records, uint32_t *tile_counter,
+                     Records records, uint32_t *tile_counter,
                      uint32_t *status, bool aligned) {
   using Smem = PartitionSmem<K, HasValues, kItems, Early, Ballots>;
   constexpr uint32_t kTile = Smem::kTile;
@@ -342,13 +406,12 @@ __global__ void __launch_bounds__(kBlock, (min_blocks<kItems, K>()))
   auto digit = [&](uint32_t i) { return (digits[i / 4] >> (8 * (i % 4))) & 0xffu; };
   uint32_t rank2[(kItems + 1) / 2]; // ranks within the warp's keys of a digit, 16 bits each
 
-  uint32_t *rec = records + static_cast<size_t>(tile) * kBins + t;
   if (Early) {
 #pragma unroll
     for (uint32_t i = 0; i < kItems; ++i)
       if (valid(i)) atomicAdd(&s.count[digit(i)], 1u);
     __syncthreads();
-    st_relaxed_u32(rec, (tile == 0 ? kRecInc : kRecAgg) | s.count[t]);
+    publish_count(records, tile, t, s.count[t]);
   }
 
   // Rank each key among the warp's earlier keys of its digit (stable: the
@@ -423,7 +486,7 @@ __global__ void __launch_bounds__(kBlock, (min_blocks<kItems, K>()))
     wc[w] = s.warp_base[w][t];
     tile_count += wc[w];
   }
-  if (!Early) st_relaxed_u32(rec, (tile == 0 ? kRecInc : kRecAgg) | tile_count);
+  if (!Early) publish_count(records, tile, t, tile_count);
   const uint32_t digit_off = block_exclusive_256(tile_count, s.tmp);
   {
     uint32_t run = digit_off;
@@ -489,7 +552,19 @@ vx_status sort_pairs(K *keys, uint32_t *values, uint32_t count,
   if (workspace == nullptr || ws_bytes < workspace_bytes<K>(count, passes))
     return VX_ERR_INVALID_VALUE;
   const Layout l = carve<K>(workspace, count, passes);
-  VX_TRY_CUDA(cudaMemsetAsync(workspace, 0, l.clear_bytes, stream));
+
+  const bool large = tune::get(sizeof(K) == 4 ? tune::kSortItemsU32 : tune::kSortItemsU64) ==
+                     static_cast<int64_t>(Shape<K>::kLarge);
+  const bool early = tune::get(tune::kSortEarlyCounts) != 0;
+  const bool ballots = tune::get(tune::kSortRankBallots) != 0;
+  const uint32_t items = large ? Shape<K>::kLarge : Shape<K>::kSmall;
+  const uint32_t tiles = ceil_div(count, kBlock * items);
+  const size_t pass_words = static_cast<size_t>(record_rows(tiles)) * kBins;
+  // the counters, the histograms and the records of this call's tiles
+  VX_TRY_CUDA(cudaMemsetAsync(workspace, 0,
+                              static_cast<size_t>(reinterpret_cast<char *>(l.records + passes * pass_words) -
+                                                  static_cast<char *>(workspace)),
+                              stream));
 
   PassInfo info{};
   for (uint32_t p = 0; p < passes; ++p) {
@@ -506,17 +581,11 @@ vx_status sort_pairs(K *keys, uint32_t *values, uint32_t count,
   }
   VX_TRY_CUDA(cudaGetLastError());
 
-  const bool large = tune::get(sizeof(K) == 4 ? tune::kSortItemsU32 : tune::kSortItemsU64) ==
-                     static_cast<int64_t>(Shape<K>::kLarge);
-  const bool early = tune::get(tune::kSortEarlyCounts) != 0;
-  const bool ballots = tune::get(tune::kSortRankBallots) != 0;
-  const uint32_t items = large ? Shape<K>::kLarge : Shape<K>::kSmall;
-  const uint32_t tiles = ceil_div(count, kBlock * items);
   K *src_k = keys, *dst_k = static_cast<K *>(l.tmp_keys);
   uint32_t *src_v = values, *dst_v = l.tmp_vals;
   auto aligned16 = [](const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
   for (uint32_t p = 0; p < passes; ++p) {
-    uint32_t *rec = l.records + static_cast<size_t>(p) * tiles * kBins;
+    const Records rec = records_of(l.records + p * pass_words, tiles);
     prof::Scope scope(sizeof(K) == 4 ? "sort_partition_u32" : "sort_partition_u64", stream);
     const bool aligned = aligned16(src_k) && (values == nullptr || aligned16(src_v));
     auto launch = [&](auto kernel, size_t smem) {
