@@ -469,8 +469,9 @@ struct WarpLeaves {
   uint8_t changed[kWarp];  // the item has a child with a new ref
 };
 
-template <int MinBlocks, bool Prefetch>
-__global__ void __launch_bounds__(kBlock, MinBlocks) leafparent_kernel(Ctx x) {
+// Climb: as in leafparent_body.
+template <bool Prefetch, bool Climb>
+__device__ __forceinline__ void leafparent_warps(const Ctx &x, Blocks blk) {
   __shared__ WarpLeaves s_warp[kBlock / kWarp];
   Header *h = x.t.hdr;
   const uint32_t l = x.t.depth - 1;
@@ -481,8 +482,8 @@ __global__ void __launch_bounds__(kBlock, MinBlocks) leafparent_kernel(Ctx x) {
   const uint32_t lane = lane_id();
   WarpLeaves &s = s_warp[threadIdx.x / kWarp];
   const DagTree tree{x.t};
-  const uint32_t stride = gridDim.x * kBlock;
-  for (uint64_t w0 = blockIdx.x * uint64_t(kBlock) + threadIdx.x - lane; w0 < W; w0 += stride) {
+  const uint32_t stride = blk.count * kBlock;
+  for (uint64_t w0 = blk.id * uint64_t(kBlock) + threadIdx.x - lane; w0 < W; w0 += stride) {
     const uint32_t wi = static_cast<uint32_t>(w0) + lane;
     const bool have = w0 + lane < W;
     Item it{};
@@ -583,9 +584,15 @@ __global__ void __launch_bounds__(kBlock, MinBlocks) leafparent_kernel(Ctx x) {
         result = canon_node(x.t, l, child);
       }
       x.a.items[base + wi].result = result;
+      if (Climb) finish_upwards(x, it.result, l); // it.result: the parent's index
     }
     __syncwarp(); // the next items overwrite the warp's buffers
   }
+}
+
+template <int MinBlocks, bool Prefetch>
+__global__ void __launch_bounds__(kBlock, MinBlocks) leafparent_kernel(Ctx x) {
+  leafparent_warps<Prefetch, false>(x, launch_blocks());
 }
 
 // The rebuilt ref of one item at inner level l from its children's results.
@@ -690,6 +697,10 @@ __global__ void publish_kernel(Ctx x) {
 // Requires every block of the grid to be resident (cudaLaunchCooperativeKernel
 // checks it).
 constexpr uint32_t kSmallBigCache = 4096;
+// From this many leaf-parent items on, a warp takes 32 of them (148 blocks of
+// 8 warps hold 37,888 at once): do and undo of 128 primitives 500 -> 347 us,
+// of 256 830 -> 490 us on B200.
+constexpr uint32_t kWarpLeafItems = 24576;
 
 // With Plain, the edit's input is a voxel list (one op): the first stages
 // turn it into leaf-mask primitives (PlainPrep) in place of the sort-based
@@ -728,7 +739,11 @@ __global__ void __maxnreg__(255) small_edit_kernel(Ctx x, EditCtx e, PlainPrep p
   // The bottom-up build without level barriers: the leaf-parent items and
   // the childless items of the levels above finish their ancestors, each
   // item rebuilt by the last of its children to finish.
-  leafparent_body<false, Lanes, true>(x, blk);
+  // Many leaf-parent items: 32 a warp; fewer: their leaves over more lanes.
+  if (x.t.hdr->item_count[x.t.depth - 1] >= kWarpLeafItems)
+    leafparent_warps<false, true>(x, blk);
+  else
+    leafparent_body<false, Lanes, true>(x, blk);
   rebuild_childless_body(x, blk);
   grid.sync();
   if (blk.id == 0 && threadIdx.x == 0) {
@@ -882,7 +897,7 @@ __global__ void pack_leaf_commands_kernel(const vx_leaf_command *c, uint32_t n, 
 // ORs run over the warp by shuffles, and the run that its last entry belongs
 // to is followed past the warp's end 32 entries at a time (by the warp that
 // holds its start), so neither dense lists (runs of 64) nor heavy duplicates
-// leave one lane walking a run alone: 0.27 -> 0.08 ms for the 8.78 M
+// leave one lane walking a run alone: 0.27 -> 0.07 ms for the 8.78 M
 // voxels of a sphere of radius 128 on B200.
 template <class K, bool Commands>
 __global__ void reduce_runs_kernel(const K *keys, const uint32_t *bits,
@@ -909,13 +924,29 @@ __global__ void reduce_runs_kernel(const K *keys, const uint32_t *bits,
   const bool valid = key < outside;
   const bool start = valid && (i == 0 || prev != key);
   uint64_t mask = valid ? mask_of(i) : 0ull;
-#pragma unroll
-  for (uint32_t d = 1; d < kWarp; d <<= 1) { // equal keys lie side by side
-    const uint64_t m = __shfl_down_sync(kFullMask, mask, d);
-    const K k = __shfl_down_sync(kFullMask, key, d);
-    if (lane + d < kWarp && k == key) mask |= m;
-  }
   const uint32_t starts = __ballot_sync(kFullMask, start);
+  // Each run's OR over the warp, in its first lane: run by run while they are
+  // few (dense lists have one or two a warp), else by segmented shuffles.
+  // (The entries before the first start belong to the warp before.)
+  if (__popc(starts) <= 4) {
+    for (uint32_t left = starts; left != 0u;) {
+      const uint32_t first = __ffs(left) - 1u;
+      left &= left - 1u;
+      const uint32_t end = left ? __ffs(left) - 1u : kWarp;
+      const bool in = valid && lane >= first && lane < end;
+      const uint32_t lo = __reduce_or_sync(kFullMask, in ? static_cast<uint32_t>(mask) : 0u);
+      const uint32_t hi = __reduce_or_sync(kFullMask, in ? static_cast<uint32_t>(mask >> 32) : 0u);
+      if (lane == first) mask = (static_cast<uint64_t>(hi) << 32) | lo;
+    }
+  } else {
+    const uint32_t after = lane == kWarp - 1 ? 0u : starts & ~((2u << lane) - 1u);
+    const uint32_t end = after ? __ffs(after) - 1u : kWarp;
+#pragma unroll
+    for (uint32_t d = 1; d < kWarp; d <<= 1) {
+      const uint64_t m = __shfl_down_sync(kFullMask, mask, d);
+      if (lane + d < end) mask |= m;
+    }
+  }
   const K last = __shfl_sync(kFullMask, key, kWarp - 1);
   const uint32_t owner = starts ? 31u - __clz(starts) : 0u;
   if (starts && last < outside && __shfl_sync(kFullMask, key, owner) == last) {
@@ -930,7 +961,7 @@ __global__ void reduce_runs_kernel(const K *keys, const uint32_t *bits,
     if (lane == owner) mask |= (static_cast<uint64_t>(hi) << 32) | lo;
   }
   if (i >= n) return;
-  const uint32_t at = offsets[i];
+  const uint32_t at = start || i == n - 1 ? offsets[i] : 0u;
   if (start) {
     vx_primitive p{};
     p.c[0] = static_cast<int32_t>(compact3(key) * 4u);

@@ -997,8 +997,8 @@ __global__ void __launch_bounds__(kBlock, 4) expand_warp_kernel(EditCtx x, Polic
 // Walking the lists costs time in proportion to the list at every level whose
 // cells hold most of it, on one block per cell: the 144,000 leaves of a
 // sphere of radius 128 in a 4096^3 world took expand_big_kernel 5.8 ms (and
-// expand_kernel 0.18 ms) of an edit's 7.0 ms on B200, the searches 0.13 ms:
-// a chain of log2(list) loads per level, in L2.
+// expand_kernel 0.18 ms) of an edit's 7.0 ms on B200, the searches 0.10 ms (by
+// halves 0.13): a chain of log8(list) round trips to L2 per level.
 template <class Policy>
 __device__ __forceinline__ void expand_sorted_body(EditCtx x, Policy pol, uint32_t l, Blocks blk) {
   Header *h = x.hdr;
@@ -1028,16 +1028,21 @@ __device__ __forceinline__ void expand_sorted_body(EditCtx x, Policy pol, uint32
       // first primitive whose key is at or after child c's first leaf
       const uint64_t want = ((keys[it.pstart] >> item_shift) << item_shift) |
                             (static_cast<uint64_t>(c) << (item_shift - 3u));
+      // Seven probes a round, loaded together: a third of a binary search's
+      // chain of round trips on the long lists of the top levels.
       lo = it.pstart;
       uint32_t n = it.pcount;
       while (n != 0) {
-        const uint32_t half = n / 2u;
-        if (keys[lo + half] < want) {
-          lo += half + 1u;
-          n -= half + 1u;
-        } else {
-          n = half;
-        }
+        const uint32_t step = n / 8u + 1u; // probes at lo + step - 1, lo + 2 step - 1, ...
+        uint64_t k[7];
+#pragma unroll
+        for (uint32_t j = 0; j < 7; ++j)
+          k[j] = (j + 1) * step <= n ? keys[lo + (j + 1) * step - 1] : ~0ull;
+        uint32_t below = 0; // probes below `want` (they ascend)
+#pragma unroll
+        for (uint32_t j = 0; j < 7; ++j) below += k[j] < want ? 1u : 0u;
+        lo += below * step;
+        n = min(n - below * step, step - 1u);
       }
     }
     const uint32_t next = __shfl_down_sync(kFullMask, lo, 1, 8);
