@@ -518,6 +518,10 @@ __device__ __forceinline__ void leafparent_warps(const Ctx &x, Blocks blk) {
         } else {
           touched = other_children(x.prims + pidx, it.cell, 4u) & 0xffu;
         }
+        const uint32_t cv = tree.const_value(pr, 0, 4);
+#pragma unroll
+        for (uint32_t c = 0; c < 8; ++c) // a leaf that holds the value already (LeftValue)
+          if (old_child[c] == cv) touched &= ~(1u << c);
       } else if (it.pcount > 1) {
         touched = 0xffu;
       }

@@ -552,6 +552,23 @@ __device__ __forceinline__ void plain_prep_fill(const PlainPrep &p, Blocks blk) 
   }
 }
 
+// The value that a child's remaining primitives leave in the voxels they
+// cover (full, empty or, with materials, one material), while it is the same
+// for all.  When the child holds that value everywhere already (added to solid
+// ground, removed from air), nothing below it changes: the child is left
+// alone and no item goes down.  Half of the items of a sphere batch on
+// terrain are of that kind (24.8 -> 12.6 M leaf-parent items at 16,384
+// spheres in 16384^3).
+struct LeftValue {
+  uint32_t value = 0;
+  bool same = true;
+  __device__ __forceinline__ void add(uint32_t v, bool first) {
+    same = first || (same && v == value);
+    value = first ? v : value;
+  }
+  __device__ __forceinline__ bool all(uint32_t held) const { return same && value == held; }
+};
+
 // Top-down expansion of level l into level l + 1 (l + 1 < depth).  Eight
 // lanes per work item, one per child cell: lane c walks the item's ordered
 // primitive list once, remembering the last primitive that covers child c
@@ -606,6 +623,9 @@ __device__ __forceinline__ void expand_body(EditCtx x, Policy pol, uint32_t l, B
     // Bit k: the list's k-th primitive cuts this child partially and comes
     // after every primitive that covers it (kept for lists of up to 32).
     uint32_t partial = 0;
+    // What those primitives leave in the voxels they cover, when all leave
+    // the same: a child that holds just that everywhere needs no edit.
+    LeftValue left;
     // Eight primitives at a time: each lane of the group loads one pair and
     // its primitive (two rounds of independent loads per chunk instead of two
     // dependent loads per primitive), then every lane walks the chunk for its
@@ -641,12 +661,16 @@ __device__ __forceinline__ void expand_body(EditCtx x, Policy pol, uint32_t l, B
           cnt = 0;
           partial = 0;
         } else if (cls == VX_CELL_MIXED) {
+          left.add(pol.const_value(s_prim[group][j], oz, csize), cnt == 0);
           ++cnt;
           if (k < 32u) partial |= 1u << k;
         }
       }
       __syncwarp(gmask); // the chunk is overwritten next
     }
+    const uint32_t const_val =
+        last_full >= 0 ? pol.const_value(x.prims[last_full], oz, csize) : 0u;
+    if (!Terrain && cnt != 0 && left.all(last_full >= 0 ? const_val : old_child)) cnt = 0;
     // Prefix sums over the 8 lanes of the group.
     uint32_t inc_items =
                  (cnt != 0 || (Policy::kItemsForConst && last_full >= 0)) ? 1u : 0u,
@@ -662,8 +686,6 @@ __device__ __forceinline__ void expand_body(EditCtx x, Policy pol, uint32_t l, B
     }
     const uint32_t group_items = __shfl_sync(kFullMask, inc_items, 7, 8);
     const uint32_t group_pairs = __shfl_sync(kFullMask, inc_pairs, 7, 8);
-    const uint32_t const_val =
-        last_full >= 0 ? pol.const_value(x.prims[last_full], oz, csize) : 0u;
     const bool full_add = last_full >= 0 && const_val == 1u;
     const bool has_item = cnt != 0 || (Policy::kItemsForConst && last_full >= 0);
     const uint32_t child_mask = (__ballot_sync(kFullMask, has_item) >> gshift) & 0xffu;
@@ -715,7 +737,7 @@ __device__ __forceinline__ void expand_body(EditCtx x, Policy pol, uint32_t l, B
       if (it.pcount <= 32u) {
         // The child's list is the set bits of `partial`: independent loads
         // of the pairs, no second classification.
-        for (uint32_t bits = partial; bits != 0u; bits &= bits - 1u)
+        for (uint32_t bits = cnt ? partial : 0u; bits != 0u; bits &= bits - 1u)
           out_pairs[my_pairs + j++] = in_pairs[it.pstart + __ffs(bits) - 1u];
       } else {
         for (uint32_t k = 0; k < it.pcount && j < cnt; ++k) {
@@ -808,11 +830,15 @@ __global__ void __launch_bounds__(kBlock, 4) expand_warp_kernel(EditCtx x, Polic
         touched = tc & 0xffu;
         covered = tc >> 8;
       }
-      const uint32_t cv = covered ? pol.const_value(pr, 0, csize) : 0u;
+      const uint32_t cv = pol.const_value(pr, 0, csize);
+      uint32_t held = 0; // children that hold just that everywhere (LeftValue)
 #pragma unroll
-      for (uint32_t c = 0; c < 8; ++c) s.ref[c][lane] = (covered >> c) & 1u ? cv : ref[c];
+      for (uint32_t c = 0; c < 8; ++c) {
+        s.ref[c][lane] = (covered >> c) & 1u ? cv : ref[c];
+        if (ref[c] == cv) held |= 1u << c;
+      }
       for (uint32_t m = covered; m != 0u; m &= m - 1u) pol.replaced(l, it.old, __ffs(m) - 1u);
-      const uint32_t mixed = touched & ~covered;
+      const uint32_t mixed = touched & ~covered & ~held;
       v = mixed | (Policy::kItemsForConst ? covered : 0u) | (covered << 8) |
           (cv == 1u ? covered << 16 : 0u);
       npairs = __popc(mixed);
@@ -839,6 +865,7 @@ __global__ void __launch_bounds__(kBlock, 4) expand_warp_kernel(EditCtx x, Polic
       const uint32_t old_child = on ? pol.child(l, old, gc) : 0u;
       int32_t last_full = -1;
       uint32_t cnt = 0, partial = 0; // as in expand_body
+      LeftValue kept;
       for (uint32_t k0 = 0; k0 < pcount; k0 += 8) {
         if (k0 + gc < pcount) {
           const uint32_t p = in_pairs[pstart + k0 + gc];
@@ -856,6 +883,7 @@ __global__ void __launch_bounds__(kBlock, 4) expand_warp_kernel(EditCtx x, Polic
             cnt = 0;
             partial = 0;
           } else if (cls == VX_CELL_MIXED) {
+            kept.add(pol.const_value(s.prim[group][j], oz, csize), cnt == 0);
             ++cnt;
             if (k < 32u) partial |= 1u << k;
           }
@@ -866,6 +894,7 @@ __global__ void __launch_bounds__(kBlock, 4) expand_warp_kernel(EditCtx x, Polic
       const bool covered = last_full >= 0;
       const uint32_t cv = covered ? pol.const_value(x.prims[last_full], oz, csize) : 0u;
       if (covered) pol.replaced(l, old, gc);
+      if (cnt != 0 && kept.all(covered ? cv : old_child)) cnt = partial = 0;
       uint32_t inc = cnt;
 #pragma unroll
       for (uint32_t d = 1; d < 8; d <<= 1) {
@@ -1008,7 +1037,7 @@ __device__ __forceinline__ void expand_sorted_body(EditCtx x, Policy pol, uint32
   const uint32_t next_base = base + W;
   if (blk.id == 0 && threadIdx.x == 0) {
     h->item_off[l + 1] = next_base;
-    h->pair_count[l + 1] = h->pair_count[l]; // every leaf goes on to one child
+    h->pair_count[l + 1] = h->pair_count[l]; // a leaf goes on to one child at most
   }
   const uint64_t *keys = x.sorted_keys;
   const uint32_t item_shift = 3 * (x.depth - l);
@@ -1046,7 +1075,10 @@ __device__ __forceinline__ void expand_sorted_body(EditCtx x, Policy pol, uint32
       }
     }
     const uint32_t next = __shfl_down_sync(kFullMask, lo, 1, 8);
-    const uint32_t cnt = have ? (c == 7u ? it.pstart + it.pcount : next) - lo : 0u;
+    uint32_t cnt = have ? (c == 7u ? it.pstart + it.pcount : next) - lo : 0u;
+    // One operation for the whole list: a child that holds its value everywhere
+    // stays as it is (LeftValue).
+    if (cnt != 0 && old_child == pol.const_value(x.prims[lo], 0, 4)) cnt = 0;
     const uint32_t some = __ballot_sync(kFullMask, cnt != 0);
     const uint32_t child_mask = (some >> gshift) & 0xffu;
     uint32_t first = 0; // one atomic per warp: four items' children

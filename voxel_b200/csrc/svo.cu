@@ -411,6 +411,10 @@ __global__ void __launch_bounds__(kBlock, Mats ? 3 : 4) leafparent_kernel(EditCt
         } else {
           touched = other_children(x.prims + pidx, it.cell, 4u) & 0xffu;
         }
+        const uint32_t cv = pol.const_value(pr, 0, 4);
+#pragma unroll
+        for (uint32_t c = 0; c < 8; ++c) // a leaf that holds the value already (LeftValue)
+          if (word[c] == cv) touched &= ~(1u << c);
       } else if (it.pcount > 1) {
         touched = 0xffu;
       }
