@@ -276,6 +276,7 @@ struct Ctx {
 struct DagTree {
   Tables t;
   static constexpr bool kItemsForConst = false;
+  static constexpr uint32_t kValueBits = 0xff00u; // the operation
   __device__ uint32_t child(uint32_t l, uint32_t ref, uint32_t c) const {
     return child_ref(t, l, ref, c);
   }

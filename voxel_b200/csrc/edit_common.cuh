@@ -401,6 +401,8 @@ __device__ __forceinline__ void note_big(const EditCtx &x, uint32_t l, uint32_t 
 //   classify<Terrain>(prim, world_exp, ox, oy, oz, n);
 //   const_value(prim, oz, n)              - the content a fully covering
 //       primitive leaves in the cube at height oz of side n (1 = full);
+//   static constexpr uint32_t kValueBits  - the bits of an edit primitive's
+//       flags that decide it;
 //   replaced(l, old, c)                   - child c of `old` is overwritten
 //       by a fully covering primitive (its subtree is dropped).
 
@@ -559,14 +561,21 @@ __device__ __forceinline__ void plain_prep_fill(const PlainPrep &p, Blocks blk) 
 // alone and no item goes down.  Half of the items of a sphere batch on
 // terrain are of that kind (24.8 -> 12.6 M leaf-parent items at 16,384
 // spheres in 16384^3).
-struct LeftValue {
-  uint32_t value = 0;
+// Kept as the flag bits that decide the value (operation, material), so that
+// a primitive costs one comparison and the value is found once at the end.
+template <class Policy> struct LeftValue {
+  uint32_t bits = 0;
   bool same = true;
-  __device__ __forceinline__ void add(uint32_t v, bool first) {
-    same = first || (same && v == value);
-    value = first ? v : value;
+  __device__ __forceinline__ void add(const vx_primitive &p, bool first) {
+    const uint32_t b = p.flags & Policy::kValueBits;
+    same = first || (same && b == bits);
+    bits = first ? b : bits;
   }
-  __device__ __forceinline__ bool all(uint32_t held) const { return same && value == held; }
+  __device__ __forceinline__ bool all(const Policy &pol, uint32_t held) const {
+    vx_primitive p{};
+    p.flags = bits;
+    return same && pol.const_value(p, 0, 4) == held;
+  }
 };
 
 // Top-down expansion of level l into level l + 1 (l + 1 < depth).  Eight
@@ -625,7 +634,7 @@ __device__ __forceinline__ void expand_body(EditCtx x, Policy pol, uint32_t l, B
     uint32_t partial = 0;
     // What those primitives leave in the voxels they cover, when all leave
     // the same: a child that holds just that everywhere needs no edit.
-    LeftValue left;
+    LeftValue<Policy> left;
     // Eight primitives at a time: each lane of the group loads one pair and
     // its primitive (two rounds of independent loads per chunk instead of two
     // dependent loads per primitive), then every lane walks the chunk for its
@@ -661,7 +670,7 @@ __device__ __forceinline__ void expand_body(EditCtx x, Policy pol, uint32_t l, B
           cnt = 0;
           partial = 0;
         } else if (cls == VX_CELL_MIXED) {
-          left.add(pol.const_value(s_prim[group][j], oz, csize), cnt == 0);
+          left.add(s_prim[group][j], cnt == 0);
           ++cnt;
           if (k < 32u) partial |= 1u << k;
         }
@@ -670,7 +679,7 @@ __device__ __forceinline__ void expand_body(EditCtx x, Policy pol, uint32_t l, B
     }
     const uint32_t const_val =
         last_full >= 0 ? pol.const_value(x.prims[last_full], oz, csize) : 0u;
-    if (!Terrain && cnt != 0 && left.all(last_full >= 0 ? const_val : old_child)) cnt = 0;
+    if (!Terrain && cnt != 0 && left.all(pol, last_full >= 0 ? const_val : old_child)) cnt = 0;
     // Prefix sums over the 8 lanes of the group.
     uint32_t inc_items =
                  (cnt != 0 || (Policy::kItemsForConst && last_full >= 0)) ? 1u : 0u,
@@ -865,7 +874,7 @@ __global__ void __launch_bounds__(kBlock, 4) expand_warp_kernel(EditCtx x, Polic
       const uint32_t old_child = on ? pol.child(l, old, gc) : 0u;
       int32_t last_full = -1;
       uint32_t cnt = 0, partial = 0; // as in expand_body
-      LeftValue kept;
+      LeftValue<Policy> kept;
       for (uint32_t k0 = 0; k0 < pcount; k0 += 8) {
         if (k0 + gc < pcount) {
           const uint32_t p = in_pairs[pstart + k0 + gc];
@@ -883,7 +892,7 @@ __global__ void __launch_bounds__(kBlock, 4) expand_warp_kernel(EditCtx x, Polic
             cnt = 0;
             partial = 0;
           } else if (cls == VX_CELL_MIXED) {
-            kept.add(pol.const_value(s.prim[group][j], oz, csize), cnt == 0);
+            kept.add(s.prim[group][j], cnt == 0);
             ++cnt;
             if (k < 32u) partial |= 1u << k;
           }
@@ -894,7 +903,7 @@ __global__ void __launch_bounds__(kBlock, 4) expand_warp_kernel(EditCtx x, Polic
       const bool covered = last_full >= 0;
       const uint32_t cv = covered ? pol.const_value(x.prims[last_full], oz, csize) : 0u;
       if (covered) pol.replaced(l, old, gc);
-      if (cnt != 0 && kept.all(covered ? cv : old_child)) cnt = partial = 0;
+      if (cnt != 0 && kept.all(pol, covered ? cv : old_child)) cnt = partial = 0;
       uint32_t inc = cnt;
 #pragma unroll
       for (uint32_t d = 1; d < 8; d <<= 1) {

@@ -88,6 +88,7 @@ __device__ __forceinline__ uint32_t prim_material(const vx_primitive &p, uint32_
 struct SvoTree {
   Tables t;
   static constexpr bool kItemsForConst = true;
+  static constexpr uint32_t kValueBits = 0xffff00u; // operation and material
   __device__ uint32_t child(uint32_t, uint32_t old, uint32_t c) const {
     if (old & kChild) return t.nodes[static_cast<size_t>(old & kIndex) * 8u + c];
     return old; // a uniform region's children hold the same value
