@@ -488,7 +488,9 @@ __device__ __forceinline__ bool cuckoo_claim(ulonglong2 *bucket, ulonglong2 e, u
 // active per instruction): a warp owns per_warp keys instead, and lanes whose
 // key has settled take the next ones once kCuckooRefill of them are idle.
 // 4.2 M keys at load 0.8, B200: 0.445 ms with a thread per key that read its
-// buckets twice, 0.368 ms reading them once, 0.285 ms so.
+// buckets twice, 0.368 ms reading them once, 0.298 ms so
+// (16.8 M: 1.88 -> 1.62 ms; 67.1 M, whose 1.3 GB table misses the TLB too: 10.8 ->
+// 12.0 ms, with 2 to 8 blocks per SM alike).
 constexpr uint32_t kCuckooRefill = 8, kCuckooBlocksPerSm = 5;
 
 __global__ void __launch_bounds__(kBlock, kCuckooBlocksPerSm)
