@@ -265,7 +265,11 @@ vx_status vx_itemset_count(const vx_itemset *set, uint64_t *host_count, vx_strea
  * arrays instead.  insert reports VX_HASH_INSERTED, VX_HASH_REPLACED (key
  * already present: value overwritten) or VX_HASH_OVERFLOW (eviction chain
  * exhausted: the key that was in hand at the end is dropped and reported).
- * find writes the value or VX_HASH_NOT_FOUND_VALUE. */
+ * find writes the value or VX_HASH_NOT_FOUND_VALUE.
+ * The keys of one insert are distinct.  A call may hold keys that are present
+ * and new ones, but a present key that another key's chain is moving while it
+ * is looked up counts as new and is stored twice: put the present ones first,
+ * or in a call of their own, where the order of the list does not ensure it. */
 typedef struct vx_cuckoo vx_cuckoo;
 vx_status vx_cuckoo_create(uint32_t slot_count, uint32_t max_evictions,
                            vx_cuckoo **out);

@@ -28,6 +28,7 @@
 #include "voxel_b200_device.cuh"
 
 #include <algorithm>
+#include <atomic>
 #include <new>
 
 namespace vx::hash {
@@ -71,6 +72,11 @@ struct vx_cuckoo {
   unsigned long long *dropped = nullptr;
   uint32_t slot_count = 0;
   uint32_t max_evictions = 0;
+  // No key can be in the table: set by a clear, reset by an insert.  A graph
+  // may clear or fill the table at any later time, so once a clear or an insert
+  // has been captured, nothing is known any more.
+  std::atomic<bool> empty{false};
+  std::atomic<bool> captured{false};
 };
 
 namespace vx::hash {
@@ -483,22 +489,107 @@ __device__ __forceinline__ bool cuckoo_claim(ulonglong2 *bucket, ulonglong2 e, u
   return false;
 }
 
-// Chains of moves differ in length (most keys need none, a few many), so a
-// thread per key leaves warps waiting for their longest chain (11 of 32 lanes
-// active per instruction): a warp owns per_warp keys instead, and lanes whose
-// key has settled take the next ones once kCuckooRefill of them are idle.
-// 4.2 M keys at load 0.8, B200: 0.445 ms with a thread per key that read its
-// buckets twice, 0.368 ms reading them once, 0.298 ms so
-// (16.8 M: 1.88 -> 1.62 ms; 67.1 M, whose 1.3 GB table misses the TLB too: 10.8 ->
-// 12.0 ms, with 2 to 8 blocks per SM alike).
-constexpr uint32_t kCuckooRefill = 8, kCuckooBlocksPerSm = 5;
+// A key's first try: both buckets are read at once.  A key that is there is
+// replaced in the slot that was read; a new one takes a free slot of the
+// emptier bucket, so that fewer keys have to move later.  VX_HASH_OVERFLOW:
+// not settled, to be moved on from (key, *target, *rnd).
+__device__ __forceinline__ uint32_t cuckoo_try(ulonglong2 *slots, uint32_t nb, uint64_t key,
+                                               uint32_t value, uint32_t &target, uint64_t &rnd) {
+  if (key == kEmpty || key == kDeleted) return VX_HASH_INVALID_KEY;
+  ulonglong2 *const b0 = slots + 2ull * vx_cuckoo_bucket(key, 0, nb);
+  ulonglong2 *const b1 = slots + 2ull * vx_cuckoo_bucket(key, 1, nb);
+  ulonglong2 *where = nullptr;
+  uint64_t word = 0;       // of the slot that holds the key
+  uint32_t free_slots = 0; // bit 2 * choice + slot
+#pragma unroll
+  for (uint32_t j = 0; j < 4; ++j) {
+    ulonglong2 *const p = (j < 2 ? b0 : b1) + (j & 1u);
+    const ulonglong2 v = ld_slot(p);
+    if (where == nullptr && v.x == key) {
+      where = p;
+      word = v.y;
+    }
+    if (v.x == kEmpty) free_slots |= 1u << j;
+  }
+  if (where != nullptr) {
+    const ulonglong2 seen = cas128(where, make_ulonglong2(key, word),
+                                   make_ulonglong2(key, (word & 0xffffffff00000000ull) | value));
+    // (moved, or its value changed, meanwhile: looked up again)
+    if ((seen.x == key && seen.y == word) || cuckoo_replace(slots, nb, key, value))
+      return VX_HASH_REPLACED;
+  }
+  rnd = mix64(key ^ 0x5851f42d4c957f2dull);
+  const uint32_t room0 = __popc(free_slots & 3u), room1 = __popc(free_slots >> 2);
+  target = room0 == room1 ? static_cast<uint32_t>(rnd >> 63) : (room1 > room0 ? 1u : 0u);
+#pragma unroll
+  for (uint32_t j = 0; j < 4; ++j) {
+    const uint32_t c = j < 2 ? target : 1u - target;
+    if (!((free_slots >> (2u * c + (j & 1u))) & 1u)) continue;
+    const ulonglong2 seen = cas128((c ? b1 : b0) + (j & 1u), make_ulonglong2(kEmpty, 0ull),
+                                   make_ulonglong2(key, with_choice(value, c)));
+    if (seen.x == kEmpty && seen.y == 0ull) return VX_HASH_INSERTED;
+  }
+  return VX_HASH_OVERFLOW;
+}
 
-__global__ void __launch_bounds__(kBlock, kCuckooBlocksPerSm)
+// One move of the entry in hand: into a slot of its bucket `target` that has
+// become free, else in the place of one of the bucket's two entries, which is
+// in hand next and goes to its other bucket.
+__device__ __forceinline__ uint32_t cuckoo_move(ulonglong2 *slots, uint32_t nb, ulonglong2 &cur,
+                                                uint32_t &target, uint64_t &rnd, uint32_t moves) {
+  ulonglong2 *const bucket = slots + 2ull * vx_cuckoo_bucket(cur.x, target, nb);
+  if (cuckoo_claim(bucket, cur, target)) return VX_HASH_INSERTED;
+  rnd = mix64(rnd + moves);
+  const ulonglong2 prev =
+      exch128(bucket + (rnd & 1u), make_ulonglong2(cur.x, with_choice(cur.y, target)));
+  if (prev.x == kEmpty || prev.x == cur.x) return VX_HASH_INSERTED; // free, or the same key
+  cur = prev;
+  target = 1u - (static_cast<uint32_t>(prev.y >> 32) & 1u);
+  return VX_HASH_OVERFLOW;
+}
+
+// A thread per key: the most keys in flight, which is what counts once the
+// table is far above L2.
+__global__ void __launch_bounds__(kBlock)
     cuckoo_insert_kernel(ulonglong2 *slots, uint32_t n, uint32_t max_evictions,
                          unsigned long long *dropped,
                          const uint64_t *__restrict__ keys,
                          const uint32_t *__restrict__ values, uint32_t count,
-                         uint32_t *statuses, uint32_t per_warp) {
+                         uint32_t *statuses) {
+  const uint64_t i = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x;
+  if (i >= count) return;
+  const uint32_t nb = n / 2u;
+  ulonglong2 cur = make_ulonglong2(keys[i], values ? values[i] : static_cast<uint32_t>(i));
+  uint32_t target = 0;
+  uint64_t rnd = 0;
+  uint32_t status = cuckoo_try(slots, nb, cur.x, static_cast<uint32_t>(cur.y), target, rnd);
+  for (uint32_t moves = 0; status == VX_HASH_OVERFLOW; ++moves) {
+    status = cuckoo_move(slots, nb, cur, target, rnd, moves);
+    if (status == VX_HASH_OVERFLOW && moves >= max_evictions) {
+      atomicAdd(dropped, 1ull);
+      break;
+    }
+  }
+  if (statuses) statuses[i] = status;
+}
+
+// Chains of moves differ in length (most keys need none, a few many), so a
+// thread per key leaves warps waiting for their longest chain (11 of 32 lanes
+// active per instruction).  Here a warp owns per_warp keys, and lanes whose
+// key has settled take the next ones once kCuckooRefill of them are idle.
+// Its warps work on all parts of the list at a time, so it is only for tables
+// that hold no key: keys that are there and lie before the new ones in the
+// list would be looked up while new ones move entries about, and one that is
+// in a lane's hand at that moment is not found and inserted a second time
+// (4.2 M slots, 1.7 M keys there and as many new: 6,000 of them).
+constexpr uint32_t kCuckooRefill = 8, kCuckooBlocksPerSm = 5;
+
+__global__ void __launch_bounds__(kBlock, kCuckooBlocksPerSm)
+    cuckoo_insert_refill_kernel(ulonglong2 *slots, uint32_t n, uint32_t max_evictions,
+                                unsigned long long *dropped,
+                                const uint64_t *__restrict__ keys,
+                                const uint32_t *__restrict__ values, uint32_t count,
+                                uint32_t *statuses, uint32_t per_warp) {
   const uint32_t nb = n / 2u;
   const uint64_t warp = (blockIdx.x * uint64_t(kBlock) + threadIdx.x) / kWarp;
   const uint64_t end = min(static_cast<uint64_t>(count), (warp + 1) * per_warp);
@@ -516,68 +607,18 @@ __global__ void __launch_bounds__(kBlock, kCuckooBlocksPerSm)
       next += __popc(idle);
       if (!busy && take < end) {
         mine = static_cast<uint32_t>(take);
-        const uint64_t key = keys[mine];
-        const uint32_t value = values ? values[mine] : mine;
-        uint32_t status = VX_HASH_OVERFLOW; // not settled yet
-        if (key == kEmpty || key == kDeleted) {
-          status = VX_HASH_INVALID_KEY;
-        } else {
-          // Both buckets at once: a key that is there is replaced; a new one
-          // takes a free slot of the emptier bucket, so that fewer keys have
-          // to move later.
-          ulonglong2 *const b0 = slots + 2ull * vx_cuckoo_bucket(key, 0, nb);
-          ulonglong2 *const b1 = slots + 2ull * vx_cuckoo_bucket(key, 1, nb);
-          bool present = false;
-          uint32_t free_slots = 0; // bit 2 * choice + slot
-#pragma unroll
-          for (uint32_t j = 0; j < 4; ++j) {
-            const ulonglong2 v = ld_slot((j < 2 ? b0 : b1) + (j & 1u));
-            present = present || v.x == key;
-            if (v.x == kEmpty) free_slots |= 1u << j;
-          }
-          rnd = mix64(key ^ 0x5851f42d4c957f2dull);
-          const uint32_t room0 = __popc(free_slots & 3u), room1 = __popc(free_slots >> 2);
-          target =
-              room0 == room1 ? static_cast<uint32_t>(rnd >> 63) : (room1 > room0 ? 1u : 0u);
-          if (present && cuckoo_replace(slots, nb, key, value)) {
-            status = VX_HASH_REPLACED;
-          } else {
-#pragma unroll
-            for (uint32_t j = 0; j < 4; ++j) {
-              const uint32_t c = j < 2 ? target : 1u - target;
-              if (status == VX_HASH_INSERTED || !((free_slots >> (2u * c + (j & 1u))) & 1u))
-                continue;
-              const ulonglong2 seen =
-                  cas128((c ? b1 : b0) + (j & 1u), make_ulonglong2(kEmpty, 0ull),
-                         make_ulonglong2(key, with_choice(value, c)));
-              if (seen.x == kEmpty && seen.y == 0ull) status = VX_HASH_INSERTED;
-            }
-          }
-        }
+        cur = make_ulonglong2(keys[mine], values ? values[mine] : mine);
+        const uint32_t status =
+            cuckoo_try(slots, nb, cur.x, static_cast<uint32_t>(cur.y), target, rnd);
         busy = status == VX_HASH_OVERFLOW;
-        cur = make_ulonglong2(key, value);
         moves = 0;
         if (!busy && statuses) statuses[mine] = status;
       }
     } else if (idle == kFullMask) {
       return; // no key left
     }
-    // One move of every entry in hand: into a slot that has become free, else
-    // in the place of one of the target bucket's two entries, which goes on to
-    // its other bucket.
-    if (busy) {
-      ulonglong2 *const bucket = slots + 2ull * vx_cuckoo_bucket(cur.x, target, nb);
-      uint32_t status = VX_HASH_OVERFLOW;
-      if (cuckoo_claim(bucket, cur, target)) {
-        status = VX_HASH_INSERTED;
-      } else {
-        rnd = mix64(rnd + moves);
-        const ulonglong2 prev =
-            exch128(bucket + (rnd & 1u), make_ulonglong2(cur.x, with_choice(cur.y, target)));
-        if (prev.x == kEmpty || prev.x == cur.x) status = VX_HASH_INSERTED; // free, or the same key
-        cur = prev;
-        target = 1u - (static_cast<uint32_t>(prev.y >> 32) & 1u);
-      }
+    if (busy) { // one move of every entry in hand
+      const uint32_t status = cuckoo_move(slots, nb, cur, target, rnd, moves);
       const bool out = status == VX_HASH_OVERFLOW && moves++ >= max_evictions;
       if (out) atomicAdd(dropped, 1ull);
       if (out || status == VX_HASH_INSERTED) {
@@ -588,6 +629,14 @@ __global__ void __launch_bounds__(kBlock, kCuckooBlocksPerSm)
     __syncwarp();
   }
 }
+
+// Empty tables of up to this many slots (268 MB, about twice L2) take the
+// refilling kernel.  B200, filled to load 0.8 in one call, us: 4.2 M keys, 84
+// MB: 303 refilling, 360 with a thread per key; 12.6 M, 252 MB: 970, 1,062;
+// 16.8 M, 335 MB: 1,680, 1,495; 67.1 M, 1.3 GB: 12,090, 8,270.  (A thread per
+// key that read its buckets twice: 450, 1,290, 1,880, 10,850.)  Below 1 M keys
+// the two are alike.
+constexpr uint32_t kCuckooRefillSlots = 1u << 24;
 
 __global__ void __launch_bounds__(kBlock)
     cuckoo_find_kernel(const ulonglong2 *slots, uint32_t n,
@@ -797,6 +846,18 @@ size_t vx_slab_set_bytes(const vx_slab_set *s) {
   return (static_cast<size_t>(s->bucket_count) + s->capacity) * sizeof(Slab);
 }
 
+// Whether a clear or an insert of the table has been captured, this one (on
+// st) included.
+static bool note_capture(vx_cuckoo *c, cudaStream_t st) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &status) != cudaSuccess) {
+    cudaGetLastError(); // the legacy stream beside another thread's capture
+    return true;
+  }
+  if (status != cudaStreamCaptureStatusNone) c->captured.store(true);
+  return c->captured.load();
+}
+
 vx_status vx_cuckoo_create(uint32_t slot_count, uint32_t max_evictions,
                            vx_cuckoo **out) {
   if (out == nullptr || slot_count == 0 || slot_count > 0xfffffffeu) return VX_ERR_INVALID_VALUE;
@@ -834,6 +895,7 @@ vx_status vx_cuckoo_clear(vx_cuckoo *c, vx_stream stream) {
   vx::prof::Scope scope("cuckoo_init", st);
   cuckoo_init_kernel<<<grid_for(c->slot_count), kBlock, 0, st>>>(
       c->slots, c->slot_count, c->dropped);
+  c->empty.store(!note_capture(c, st));
   return vx::from_cuda(cudaGetLastError());
 }
 
@@ -844,14 +906,20 @@ vx_status vx_cuckoo_insert(vx_cuckoo *c, const uint64_t *keys,
   if (count == 0) return VX_OK;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   vx::prof::Scope scope("cuckoo_insert", st);
+  const bool captured = note_capture(c, st);
+  if (!c->empty.exchange(false) || captured || c->slot_count > kCuckooRefillSlots) {
+    cuckoo_insert_kernel<<<vx::ceil_div(count, kBlock), kBlock, 0, st>>>(
+        c->slots, c->slot_count, c->max_evictions, c->dropped, keys, values, count, statuses);
+    return vx::from_cuda(cudaGetLastError());
+  }
   // As many warps as are resident at once, 32 keys each at least.
   const uint32_t warps =
       static_cast<uint32_t>(vx::sm_count()) * kCuckooBlocksPerSm * (kBlock / vx::kWarp);
   const uint32_t per_warp = std::max(vx::kWarp, vx::ceil_div(count, warps));
   const uint32_t blocks = vx::ceil_div(vx::ceil_div(count, per_warp), kBlock / vx::kWarp);
-  cuckoo_insert_kernel<<<blocks, kBlock, 0, st>>>(c->slots, c->slot_count, c->max_evictions,
-                                                  c->dropped, keys, values, count, statuses,
-                                                  per_warp);
+  cuckoo_insert_refill_kernel<<<blocks, kBlock, 0, st>>>(
+      c->slots, c->slot_count, c->max_evictions, c->dropped, keys, values, count, statuses,
+      per_warp);
   return vx::from_cuda(cudaGetLastError());
 }
 
