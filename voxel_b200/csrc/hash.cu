@@ -865,7 +865,7 @@ vx_status vx_cuckoo_create(uint32_t slot_count, uint32_t max_evictions,
   if (c == nullptr) return VX_ERR_MEMORY_ALLOCATION;
   c->slot_count = std::max<uint32_t>(2u, (slot_count + 1u) & ~1u); // whole two-slot buckets
   c->max_evictions = max_evictions;
-  cudaError_t e = cudaMalloc(&c->slots, sizeof(ulonglong2) * slot_count);
+  cudaError_t e = cudaMalloc(&c->slots, sizeof(ulonglong2) * c->slot_count);
   if (e == cudaSuccess) e = cudaMalloc(&c->dropped, sizeof(unsigned long long));
   if (e != cudaSuccess) {
     vx_cuckoo_destroy(c);
