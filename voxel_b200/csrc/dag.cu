@@ -767,38 +767,92 @@ __global__ void query_kernel(vx_dag_view v, const vx_voxel *pts, uint32_t n,
 }
 
 // Rays differ in length by orders of magnitude (a miss of the world, a ray
-// along a cave), so a thread per ray leaves a warp waiting for its longest:
-// 5.75 of 32 lanes were active per instruction.  A warp owns per_warp rays
-// instead, and lanes whose ray has ended take the next ones once kRayRefill
-// of them are idle.  The cells that a ray's path goes through are kept in a
-// column of shared memory per thread.  1 M rays (half downwards on the
-// terrain, half at random) on a 4096^3 DAG, B200: 0.86 -> 0.65 ms, now bound
-// by the longest rays (65,536 rays alone take 0.32 ms): refills of 16 lanes
-// take 0.69 ms, 8 steps between refills 0.78 ms, two or three times as many
-// warps 0.77-0.83 ms, walks of at most 1-3 levels a step 0.75-0.93 ms.
+// along a cave).  Two kernels share a list of rays, 32 at a time:
+//
+// raycast_kernel, a thread per ray, takes those whose 32 rays are alike
+// (primary rays of neighbouring pixels): they walk the same cells, so the
+// warp stays together, and its blocks are dealt out as others end.
+//
+// raycast_refill_kernel takes the others.  A thread per ray would leave a warp
+// waiting for its longest (5.75 of 32 lanes were active per instruction), so
+// a warp takes rays from its share as its lanes' rays end, once kRayRefill
+// lanes are idle.  Shares are every so-many-th 32 rays: neighbours in the list
+// cost alike.  The cells that a ray's path goes through are kept in a column
+// of shared memory per thread.
+//
+// B200, a 4096^3 DAG, us, a thread per ray / refilling / both kernels as here:
+//   1 M rays, half downwards on the terrain, half at random   801 / 590 / 613
+//   images of 1024^2 rays from three eyes  393 530 293 / 461 713 305 / 416 548 302
+//   images of 2048^2 rays                861 1442 520 / 1221 2079 698 / 900 1490 575
+//   65,536 rays                                               209 / 225 / -
+// Up to kRayFewest rays, which all run at once, are alike for this purpose:
+// the longest decides.  (Refilling at 16 and 24 idle lanes, 2 and 8 steps
+// between refills, 4 and 6 blocks per SM: 600-800 us for the first.)
 constexpr uint32_t kRayRefill = 8, kRaySteps = 4, kRayBlocksPerSm = 5;
+constexpr uint32_t kRayFewest = 1u << 17;
+
+// Whether the 32 rays from `first` on are alike: directions within 11.5 degrees
+// (cos^2 0.96) of the first one's and origins within a sixteenth of the world
+// of its origin; fewer than 32 rays are.  Called by a whole warp.  Rounded
+// operations throughout, so that both kernels find the same.
+__device__ __forceinline__ bool rays_alike(const vx_ray *rays, uint64_t first, uint32_t n,
+                                           float reach) {
+  if (first + kWarp > n) return true;
+  const vx_ray r = rays[first + lane_id()];
+  float dot = 0.0f, mine = 0.0f, lead = 0.0f;
+  bool near = true;
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    const float d0 = __shfl_sync(kFullMask, r.dir[a], 0);
+    const float o0 = __shfl_sync(kFullMask, r.origin[a], 0);
+    dot = __fadd_rn(dot, __fmul_rn(r.dir[a], d0));
+    mine = __fadd_rn(mine, __fmul_rn(r.dir[a], r.dir[a]));
+    lead = __fadd_rn(lead, __fmul_rn(d0, d0));
+    near = near && fabsf(__fsub_rn(r.origin[a], o0)) <= reach;
+  }
+  const bool aligned =
+      dot > 0.0f && __fmul_rn(dot, dot) >= __fmul_rn(0.96f, __fmul_rn(mine, lead));
+  return __all_sync(kFullMask, near && aligned);
+}
+
+// All: every ray; otherwise those that rays_alike names.
+template <bool All>
+__global__ void __launch_bounds__(kBlock)
+    raycast_kernel(vx_dag_view v, const vx_ray *rays, uint32_t n, vx_ray_hit *hits, float reach) {
+  const uint64_t i = blockIdx.x * uint64_t(kBlock) + threadIdx.x;
+  if (i - lane_id() >= n) return;
+  if (!All && !rays_alike(rays, i - lane_id(), n, reach)) return;
+  if (i < n) hits[i] = vx_dag_raycast(v, rays[i]);
+}
 
 __global__ void __launch_bounds__(kBlock, kRayBlocksPerSm)
-    raycast_kernel(vx_dag_view v, const vx_ray *rays, uint32_t n, vx_ray_hit *hits,
-                   uint32_t per_warp) {
+    raycast_refill_kernel(vx_dag_view v, const vx_ray *rays, uint32_t n, vx_ray_hit *hits,
+                          float reach) {
   __shared__ uint32_t s_path[kMaxDepth + 1][kBlock];
   uint32_t *path = &s_path[0][threadIdx.x];
-  const uint64_t warp = (blockIdx.x * uint64_t(kBlock) + threadIdx.x) / kWarp;
-  const uint64_t end = min(static_cast<uint64_t>(n), (warp + 1) * per_warp);
-  uint64_t next = warp * per_warp; // the same on the warp's lanes
+  const uint64_t stride = gridDim.x * uint64_t(kBlock);
+  // the warp's current 32 rays and how many of them are taken
+  uint64_t first = blockIdx.x * uint64_t(kBlock) + threadIdx.x - lane_id();
+  uint32_t taken = 0;
+  while (first < n && rays_alike(rays, first, n, reach)) first += stride;
   vx_dag_ray ray;
-  uint32_t mine = 0;
+  uint64_t mine = 0;
   bool active = false;
   for (;;) {
     const uint32_t idle = __ballot_sync(kFullMask, !active);
-    if (next < end && __popc(idle) >= kRayRefill) {
-      const uint64_t take = next + __popc(idle & lanemask_lt());
-      if (!active && take < end) {
-        mine = static_cast<uint32_t>(take);
+    if (first < n && __popc(idle) >= kRayRefill) {
+      const uint32_t take = taken + __popc(idle & lanemask_lt());
+      if (!active && take < kWarp) {
+        mine = first + take;
         active = vx_dag_ray_begin(v, rays[mine], ray, path);
         if (!active) hits[mine] = vx_ray_miss();
       }
-      next += __popc(idle);
+      taken += __popc(idle);
+      if (taken >= kWarp) { // (some idle lanes may wait for the next round)
+        taken = 0;
+        do first += stride;
+        while (first < n && rays_alike(rays, first, n, reach));
+      }
     } else if (idle == kFullMask) {
       return; // no ray left
     }
@@ -1553,12 +1607,16 @@ vx_status vx_dag_raycast(const vx_dag *d, const vx_ray *rays, uint32_t count,
   vx::prof::Scope sc("dag_raycast", s);
   vx_dag_view view;
   VX_TRY(vx_dag_device_view(d, &view));
-  // As many warps as are resident at once, 32 rays each at least.
-  const uint32_t warps =
-      static_cast<uint32_t>(vx::sm_count()) * kRayBlocksPerSm * (kBlock / vx::kWarp);
-  const uint32_t per_warp = std::max(vx::kWarp, vx::ceil_div(count, warps));
-  const uint32_t blocks = vx::ceil_div(vx::ceil_div(count, per_warp), kBlock / vx::kWarp);
-  raycast_kernel<<<blocks, kBlock, 0, s>>>(view, rays, count, hits, per_warp);
+  const uint32_t blocks = vx::ceil_div(count, kBlock);
+  const float reach = static_cast<float>(4u << view.depth) / 16.0f;
+  if (count <= kRayFewest) {
+    raycast_kernel<true><<<blocks, kBlock, 0, s>>>(view, rays, count, hits, reach);
+    return vx::from_cuda(cudaGetLastError());
+  }
+  raycast_kernel<false><<<blocks, kBlock, 0, s>>>(view, rays, count, hits, reach);
+  VX_TRY_CUDA(cudaGetLastError());
+  raycast_refill_kernel<<<std::min(blocks, static_cast<uint32_t>(vx::sm_count()) * kRayBlocksPerSm),
+                          kBlock, 0, s>>>(view, rays, count, hits, reach);
   return vx::from_cuda(cudaGetLastError());
 }
 
