@@ -597,7 +597,9 @@ __device__ __forceinline__ void leafparent_warps(const Ctx &x, Blocks blk) {
 
 template <int MinBlocks, bool Prefetch>
 __global__ void __launch_bounds__(kBlock, MinBlocks) leafparent_kernel(Ctx x) {
-  leafparent_warps<Prefetch, false>(x, launch_blocks());
+  if (x.t.hdr->item_count[x.t.depth - 1] <= kWideItems)
+    leafparent_body<false, 8>(x, launch_blocks());
+  else leafparent_warps<Prefetch, false>(x, launch_blocks());
 }
 
 // The rebuilt ref of one item at inner level l from its children's results.
@@ -702,6 +704,7 @@ __global__ void publish_kernel(Ctx x) {
 // Requires every block of the grid to be resident (cudaLaunchCooperativeKernel
 // checks it).
 constexpr uint32_t kSmallBigCache = 4096;
+
 // From this many leaf-parent items on, a warp takes 32 of them (148 blocks of
 // 8 warps hold 37,888 at once): do and undo of 128 primitives 500 -> 347 us,
 // of 256 830 -> 490 us on B200.
@@ -1153,7 +1156,7 @@ vx_status run_pipeline(vx_dag *d, const vx_primitive *prims,
         expand_sorted_kernel<DagTree><<<lgrid, kBlock, 0, s>>>(e, tree, l);
       else
         expand_warp_kernel<DagTree>
-            <<<level_grid(grid, l, kBlock), kBlock, 0, s>>>(e, tree, l);
+            <<<lgrid, kBlock, 0, s>>>(e, tree, l);
     }
     VX_TRY_CUDA(cudaGetLastError());
     if (sorted_keys != nullptr || terrain) continue; // no long lists

@@ -771,6 +771,17 @@ __global__ void __launch_bounds__(kBlock)
   expand_body<Policy, Terrain>(x, pol, l, launch_blocks());
 }
 
+// Up to this many items a level's batch kernels (expand, leaf parents) give
+// eight lanes to an item instead of one: so many are on the chip at once, and
+// a warp that takes 32 items with several primitives each would walk their
+// lists four (expansion) or a leaf at a time (leaf parents) while most of the
+// chip has nothing to do.  B200, us, one lane / eight lanes up to here (eight
+// always): 2,000 spheres of radius 16-64 with their centres in a 256^3 part
+// of a 2048^3 Hash DAG 620 / 377 (453), of an SVO 578 / 390 (594); 1,000
+// primitives in a 256^3 world 393 / 187 (287); 8,000 spheres all over 2048^3
+// 592 / 470 (893).
+constexpr uint32_t kWideItems = 37888; // 148 multiprocessors x 256 groups of eight
+
 // expand_body for the batches' own launches: a warp takes 32 items at a time
 // with no block barrier.  At the levels that hold most items nearly every
 // list is one primitive (at 16,384 spheres in 16384^3, 6.67 M primitives for
@@ -800,6 +811,10 @@ __global__ void __launch_bounds__(kBlock, 4) expand_warp_kernel(EditCtx x, Polic
   Header *h = x.hdr;
   const uint32_t W = h->item_count[l]; // loaded beside the status
   const uint32_t base = h->item_off[l];
+  if (W <= kWideItems) { // the same in every block
+    expand_body<Policy, false>(x, pol, l, launch_blocks());
+    return;
+  }
   if (edit_failed(h)) return;
   const uint32_t depth = x.depth;
   const uint32_t next_base = base + W;

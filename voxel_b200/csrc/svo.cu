@@ -377,6 +377,10 @@ __global__ void __launch_bounds__(kBlock, Mats ? 3 : 4) leafparent_kernel(EditCt
   const uint32_t W = h->item_count[l]; // loaded beside the status
   const uint32_t base = h->item_off[l];
   if (edit_failed(h)) return;
+  if (W <= kWideItems) { // the same in every block
+    leafparent_body<false>(x, t, launch_blocks());
+    return;
+  }
   const uint32_t *pairs = x.a.pairs[l & 1u];
   const uint32_t lane = lane_id();
   WarpCells &s = s_warp[threadIdx.x / kWarp];
@@ -1043,7 +1047,7 @@ vx_status run_pipeline(vx_svo *v, const vx_primitive *prims, const uint32_t *d_c
       else if (sorted_keys) expand_sorted_kernel<SvoTree><<<lgrid, kBlock, 0, s>>>(e, pol, l);
       else
         expand_warp_kernel<SvoTree>
-            <<<level_grid(grid, l, kBlock), kBlock, 0, s>>>(e, pol, l);
+            <<<lgrid, kBlock, 0, s>>>(e, pol, l);
     }
     VX_TRY_CUDA(cudaGetLastError());
     if (sorted_keys != nullptr || terrain) continue; // no long lists
