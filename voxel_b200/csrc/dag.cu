@@ -666,23 +666,21 @@ __device__ void finish_upwards(const Ctx &x, uint32_t parent, uint32_t l) {
 // start their own climb.
 __device__ __forceinline__ void rebuild_childless_body(Ctx x, Blocks blk) {
   Header *h = x.t.hdr;
-  // every level's counts in one round trip
-  __shared__ uint32_t s_w[kMaxDepth], s_base[kMaxDepth];
-  if (threadIdx.x < kMaxDepth) {
-    s_w[threadIdx.x] = h->item_count[threadIdx.x];
-    s_base[threadIdx.x] = h->item_off[threadIdx.x];
-  }
-  if (edit_failed(h)) return; // (its barrier also publishes s_w, s_base)
-  for (uint32_t l = 0; l + 1 < x.t.depth; ++l) {
-    const uint32_t W = s_w[l];
-    const uint32_t base = s_base[l];
-    for (uint64_t i = blk.id * static_cast<uint64_t>(blockDim.x) + threadIdx.x;
-         i < W; i += static_cast<uint64_t>(blk.count) * blockDim.x) {
-      const Item it = x.a.items[base + i];
-      if (it.masks & 0xffu) continue;
-      x.a.items[base + i].result = build_item<false, true>(x, l, it);
-      finish_upwards(x, it.result, l);
-    }
+  // Every level's first item, in one round trip.  The levels' items lie one
+  // after the other, so one thread takes one item of any level and the climbs
+  // run side by side; level by level they had to wait for one another.
+  __shared__ uint32_t s_base[kMaxDepth];
+  if (threadIdx.x < kMaxDepth) s_base[threadIdx.x] = h->item_off[threadIdx.x];
+  if (edit_failed(h)) return; // (its barrier also publishes s_base)
+  const uint32_t n = s_base[x.t.depth - 1]; // the first leaf-parent item
+  for (uint64_t i = blk.id * static_cast<uint64_t>(blockDim.x) + threadIdx.x; i < n;
+       i += static_cast<uint64_t>(blk.count) * blockDim.x) {
+    const Item it = x.a.items[i];
+    if (it.masks & 0xffu) continue;
+    uint32_t l = 0;
+    while (l + 2 < x.t.depth && s_base[l + 1] <= i) ++l;
+    x.a.items[i].result = build_item<false, true>(x, l, it);
+    finish_upwards(x, it.result, l);
   }
 }
 
@@ -752,7 +750,8 @@ __global__ void __maxnreg__(255) small_edit_kernel(Ctx x, EditCtx e, PlainPrep p
     leafparent_warps<false, true>(x, blk);
   else
     leafparent_body<false, Lanes, true>(x, blk);
-  rebuild_childless_body(x, blk);
+  // (from the last block down: the leaf-parent items start at the first)
+  rebuild_childless_body(x, Blocks{blk.count - 1u - blk.id, blk.count});
   grid.sync();
   if (blk.id == 0 && threadIdx.x == 0) {
     Header *h = x.t.hdr;

@@ -598,23 +598,21 @@ __device__ void finish_upwards(const EditCtx &x, const Tables &t, uint32_t paren
 // start their own climb.
 __device__ __forceinline__ void rebuild_childless_body(EditCtx x, Tables t, Blocks blk) {
   Header *h = x.hdr;
-  // every level's counts in one round trip
-  __shared__ uint32_t s_w[kMaxDepth], s_base[kMaxDepth];
-  if (threadIdx.x < kMaxDepth) {
-    s_w[threadIdx.x] = h->item_count[threadIdx.x];
-    s_base[threadIdx.x] = h->item_off[threadIdx.x];
-  }
-  if (edit_failed(h)) return; // (its barrier also publishes s_w, s_base)
-  for (uint32_t l = 0; l + 1 < t.depth; ++l) {
-    const uint32_t W = s_w[l];
-    const uint32_t base = s_base[l];
-    for (uint64_t i = blk.id * static_cast<uint64_t>(blockDim.x) + threadIdx.x;
-         i < W; i += static_cast<uint64_t>(blk.count) * blockDim.x) {
-      const Item it = x.a.items[base + i];
-      if (it.masks & 0xffu) continue;
-      x.a.items[base + i].result = build_item<true>(x, t, l, it);
-      finish_upwards(x, t, it.result, l);
-    }
+  // Every level's first item, in one round trip.  The levels' items lie one
+  // after the other, so one thread takes one item of any level and the climbs
+  // run side by side; level by level they had to wait for one another.
+  __shared__ uint32_t s_base[kMaxDepth];
+  if (threadIdx.x < kMaxDepth) s_base[threadIdx.x] = h->item_off[threadIdx.x];
+  if (edit_failed(h)) return; // (its barrier also publishes s_base)
+  const uint32_t n = s_base[t.depth - 1]; // the first leaf-parent item
+  for (uint64_t i = blk.id * static_cast<uint64_t>(blockDim.x) + threadIdx.x; i < n;
+       i += static_cast<uint64_t>(blk.count) * blockDim.x) {
+    const Item it = x.a.items[i];
+    if (it.masks & 0xffu) continue;
+    uint32_t l = 0;
+    while (l + 2 < t.depth && s_base[l + 1] <= i) ++l;
+    x.a.items[i].result = build_item<true>(x, t, l, it);
+    finish_upwards(x, t, it.result, l);
   }
 }
 
@@ -912,7 +910,8 @@ __global__ void __maxnreg__(255) small_edit_kernel(EditCtx e, Tables t, PlainPre
   // item rebuilt by the last of its children to finish.
   if (verdict != 2u) {
     leafparent_body<false, true>(e, t, blk);
-    rebuild_childless_body(e, t, blk);
+    // (from the last block down: the leaf-parent items start at the first)
+    rebuild_childless_body(e, t, Blocks{blk.count - 1u - blk.id, blk.count});
   }
   grid.sync();
   if (lead) {
