@@ -37,11 +37,13 @@ constexpr uint32_t kWarps = kBlock / kWarp;
 constexpr uint32_t kMaxPasses = 8;
 constexpr uint32_t kMaxCount = (1u << 30) - 1u;
 
-// Items per thread of the partition kernel (the tile is 256 x items keys):
-// the small setting fits four blocks per SM (64 registers, ~35 KB of shared
-// memory each), the large one three with more keys per tile (on B200 the
-// large one is faster: 2.72 vs 3.13 ms for 2^26 u32 pairs).  The tuning
-// knobs "sort.items_u32" / "sort.items_u64" pick one per device.
+// Items per thread of the partition kernel (the tile is 256 x items keys).
+// With values and ranking by match words a block of the small setting takes 46
+// KB of shared memory, one of the large setting 55 KB: four per SM either way,
+// 64 registers a thread (by ballots the small setting takes 30 KB: five, 48
+// registers).  On B200 the large one is faster: 1.82
+// against 1.84 ms for 2^26 u32 pairs, 2.18 against 2.32 ms for 2^25 60-bit u64
+// pairs.  The tuning knobs "sort.items_u32" / "sort.items_u64" pick one per device.
 template <class K> struct Shape;
 template <> struct Shape<uint32_t> {
   static constexpr uint32_t kSmall = 12, kLarge = 16;
@@ -49,8 +51,8 @@ template <> struct Shape<uint32_t> {
 template <> struct Shape<uint64_t> {
   static constexpr uint32_t kSmall = 8, kLarge = 10;
 };
-template <uint32_t Items, class K> constexpr uint32_t min_blocks() {
-  return Items == Shape<K>::kSmall ? 5u : 4u;
+template <uint32_t Items, class K, bool Ballots> constexpr uint32_t min_blocks() {
+  return Ballots && Items == Shape<K>::kSmall ? 5u : 4u;
 }
 // Tiles of the small setting: the most tiles, so the workspace covers both.
 template <class K> inline uint32_t max_tiles(uint32_t count) {
@@ -209,7 +211,7 @@ struct PartitionSmem {
 // indices throughout, two ranks share a register, and one table gives each
 // (warp, digit) its tile-local base.
 template <class K, bool HasValues, uint32_t kItems, bool Early, bool Ballots>
-__global__ void __launch_bounds__(kBlock, (min_blocks<kItems, K>()))
+__global__ void __launch_bounds__(kBlock, (min_blocks<kItems, K, Ballots>()))
     partition_kernel(const K *__restrict__ in_keys,
                      const uint32_t *__restrict__ in_vals,
                      K *__restrict__ out_keys, uint32_t *__restrict__ out_vals,
