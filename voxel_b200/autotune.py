@@ -16,13 +16,23 @@ which the library applies when it is first loaded on that kind of device:
   * scan.tile_kb: the prefix sum's tile (32, 16 or 8 KB, with 6, 12 or 24
     resident blocks per SM); timed on 2^28 u32;
   * edit.big_item / edit.blocks_per_sm / edit.leafparent_blocks /
-    edit.leafparent_lanes / edit.leafparent_prefetch: the primitive-list
-    length above which a work item is expanded by a whole block, the grid of
-    the edit pipelines' item kernels, and the resident blocks, threads per
-    item and next-node prefetch of the DAG leaf-parent kernel; timed on the
-    batched Hash
-    DAG edit of the benchmark (16384^3 cave terrain at scale 64, 16,384
-    spheres of radius log-uniform in [1, 256], 60 % add).
+    edit.leafparent_prefetch: the primitive-list length above which a work
+    item is expanded by a block or a cluster of blocks, the grid of the edit
+    pipelines' item kernels, and the resident blocks and next-node prefetch
+    of the DAG leaf-parent kernel; timed on the batched Hash DAG edit of the
+    benchmark (16384^3 cave terrain at scale 64, 16,384 spheres of radius
+    log-uniform in [1, 256], 60 % add);
+  * edit.leafparent_lanes: the threads per leaf-parent item in small edits
+    (one cooperative launch); timed on do and undo of 1, 8, 32 and 128
+    spheres and boxes of radius up to 128 on a 2048^3 Hash DAG;
+  * edit.small_max_voxels: the longest voxel list that runs as one
+    cooperative launch; timed on lists of 2,000 to 54,000 voxels, placed in
+    and removed from a Hash DAG and an SVO: brush strokes (the voxels of a
+    sphere, which gain from it) and voxels all over the world (a leaf each,
+    which lose);
+  * serve.blocks_per_sm: the grid of the serving loop's edit graphs.
+
+A setting replaces the default only when it is more than 4 % faster.
 
 Every setting's output is compared with the default setting's (the sorted
 arrays bit for bit, the edited DAG by 2^20 point queries) before its time
@@ -58,6 +68,14 @@ def _time(fn, reps: int, before=None) -> float:
         if i:  # the first run warms up
             ts.append(a.elapsed_time(b))
     return float(np.median(ts))
+
+
+def _pick(times: dict, default):
+    """The fastest setting, or the default where nothing is faster by more
+    than the runs of one setting differ."""
+    times = {k: t for k, t in times.items() if t is not None}
+    best = min(times, key=times.get)
+    return default if default in times and times[default] <= 1.04 * times[best] else best
 
 
 def tune_sort(n32: int, n64: int, reps: int, log) -> tuple[dict, dict]:
@@ -114,13 +132,14 @@ def tune_sort(n32: int, n64: int, reps: int, log) -> tuple[dict, dict]:
             cand = [c for c in cand if c is not None]
             tot = tot + min(cand) if cand else float("inf")
         score[(early, ballots, radix)] = tot
-    early, ballots, radix = min(score, key=score.get)
+    now = vx.tuning()
+    early, ballots, radix = _pick(score, tuple(now[k] for k in (
+        "sort.early_counts", "sort.rank_ballots", "sort.radix_bits")))
     best["sort.early_counts"], best["sort.rank_ballots"] = early, ballots
     best["sort.radix_bits"] = radix
     for label, (_, _, knob) in cases.items():
         opts = {i: times[(label, i, early, ballots, radix)] for i in vx.tuning_options(knob)}
-        opts = {i: t for i, t in opts.items() if t is not None}
-        best[knob] = min(opts, key=opts.get)
+        best[knob] = _pick(opts, now[knob])
     return best, {f"{l} items={i} early={e} ballots={b} radix={r}": t
                   for (l, i, e, b, r), t in times.items()}
 
@@ -146,8 +165,8 @@ def tune_scan(n: int, reps: int, log) -> tuple[dict, dict]:
         times[f"tile_kb={kb}"] = ms
         log(f"  scan u32 tile_kb={kb}: " + (f"{ms:.3f} ms" if same else "DIFFERENT OUTPUT (not used)"))
     vx.reset_tuning()
-    valid = {int(k.split("=")[1]): t for k, t in times.items() if t is not None}
-    return {"scan.tile_kb": min(valid, key=valid.get)}, times
+    valid = {int(k.split("=")[1]): t for k, t in times.items()}
+    return {"scan.tile_kb": _pick(valid, vx.tuning()["scan.tile_kb"])}, times
 
 
 def tune_edit(depth: int, scale: int, count: int, reps: int, log, max_nodes: int,
@@ -170,11 +189,10 @@ def tune_edit(depth: int, scale: int, count: int, reps: int, log, max_nodes: int
     ref = work.query(pts)
     times: dict = {}
 
-    def measure(big, bps, lpb, lanes, pf=0):
+    def measure(big, bps, lpb, pf):
         vx.set_tuning("edit.big_item", big)
         vx.set_tuning("edit.blocks_per_sm", bps)
         vx.set_tuning("edit.leafparent_blocks", lpb)
-        vx.set_tuning("edit.leafparent_lanes", lanes)
         vx.set_tuning("edit.leafparent_prefetch", pf)
         work.copy_from(pristine)
         work.apply_primitives(prims)
@@ -184,44 +202,105 @@ def tune_edit(depth: int, scale: int, count: int, reps: int, log, max_nodes: int
         if ok and work.status() != 0:
             ms = None
         key = (f"big_item={big} blocks_per_sm={bps} leafparent_blocks={lpb} "
-               f"leafparent_lanes={lanes}" + (" leafparent_prefetch=1" if pf else ""))
+               f"leafparent_prefetch={pf}")
         times[key] = ms
         log(f"  edit {key}: "
             + (f"{ms:.3f} ms" if ms is not None else "FAILED OR DIFFERENT (not used)"))
         return ms
 
-    # Stage 1: long-list threshold and grid.  Among settings within 2 % of
-    # the fastest, take the smallest grid: on a large batch more blocks gain
-    # little, while on small batches (the serving loop's) every extra block
-    # is launch overhead.
-    lpb0 = vx.tuning()["edit.leafparent_blocks"]
-    lanes0 = vx.tuning()["edit.leafparent_lanes"]
-    stage1 = {}
-    for big, bps in itertools.product(vx.tuning_options("edit.big_item"),
-                                      vx.tuning_options("edit.blocks_per_sm")):
-        ms = measure(big, bps, lpb0, lanes0)
-        if ms is not None:
-            stage1[(big, bps)] = ms
-    fastest = min(stage1.values())
-    near = [k for k, t in stage1.items() if t <= 1.02 * fastest]
-    big, bps = min(near, key=lambda k: (k[1], stage1[k]))
-    # Stage 2: threads per item, resident blocks and next-node prefetch of
-    # the leaf-parent kernel at that setting (the prefetch form exists for 4
-    # threads per item).
-    stage2 = {}
-    for lpb, lanes, pf in itertools.product(vx.tuning_options("edit.leafparent_blocks"),
-                                            vx.tuning_options("edit.leafparent_lanes"),
-                                            vx.tuning_options("edit.leafparent_prefetch")):
-        if pf and lanes != 4:
-            continue
-        ms = measure(big, bps, lpb, lanes, pf)
-        if ms is not None:
-            stage2[(lpb, lanes, pf)] = ms
-    lpb, lanes, pf = min(stage2, key=stage2.get)
+    # Stage 1: long-list threshold and grid.
+    now = vx.tuning()
+    lpb0, pf0 = now["edit.leafparent_blocks"], now["edit.leafparent_prefetch"]
+    stage1 = {(big, bps): measure(big, bps, lpb0, pf0)
+              for big, bps in itertools.product(vx.tuning_options("edit.big_item"),
+                                                vx.tuning_options("edit.blocks_per_sm"))}
+    big, bps = _pick(stage1, (now["edit.big_item"], now["edit.blocks_per_sm"]))
+    # Stage 2: resident blocks and next-node prefetch of the leaf-parent
+    # kernel at that setting.
+    stage2 = {(lpb, pf): measure(big, bps, lpb, pf)
+              for lpb, pf in itertools.product(vx.tuning_options("edit.leafparent_blocks"),
+                                               vx.tuning_options("edit.leafparent_prefetch"))}
+    lpb, pf = _pick(stage2, (lpb0, pf0))
     vx.reset_tuning()
     return {"edit.big_item": big, "edit.blocks_per_sm": bps,
-            "edit.leafparent_blocks": lpb, "edit.leafparent_lanes": lanes,
-            "edit.leafparent_prefetch": pf}, times
+            "edit.leafparent_blocks": lpb, "edit.leafparent_prefetch": pf}, times
+
+
+def _geomean(ts) -> float:
+    return float(np.exp(np.mean(np.log(ts))))
+
+
+def tune_small(depth: int, scale: int, strokes, reps: int, log, max_nodes: int,
+               arena: int) -> tuple[dict, dict]:
+    """edit.leafparent_lanes and edit.small_max_voxels: geometric means over
+    small edits and over voxel lists; each setting's result is compared by
+    point queries with the default's."""
+    g = torch.Generator(device="cuda")
+    g.manual_seed(14)
+    pts = torch.randint(0, 4 << depth, (1 << 18, 3), dtype=torch.int32, device="cuda",
+                        generator=g)
+    dag = vx.HashDag(depth, max_nodes, arena)
+    dag.build_terrain(7, scale, True)
+    svo = vx.Svo(depth, 2 * max_nodes, 8 * max_nodes, arena_bytes=arena)
+    svo.build_terrain(7, scale, True)
+    if dag.status() != 0 or svo.status() != 0:
+        raise RuntimeError("terrain build failed")
+    times: dict = {}
+    now = vx.tuning()
+
+    def sweep(knob, calls, look):
+        """calls: {name: fn}; look(): what the calls leave, to compare."""
+        ref, means = None, {}
+        for v in [now[knob]] + [v for v in vx.tuning_options(knob) if v != now[knob]]:
+            vx.set_tuning(knob, v)
+            ts = []
+            for name, fn in calls.items():
+                ts.append(_time(fn, reps))
+                times[f"{knob}={v} {name}"] = ts[-1]
+            got = look()
+            ref = got if ref is None else ref
+            means[v] = _geomean(ts) if torch.equal(got, ref) else None
+            log(f"  {knob}={v}: "
+                + (f"{means[v]:.4f} ms" if means[v] is not None else "DIFFERENT (not used)"))
+        vx.reset_tuning()
+        return _pick(means, now[knob])
+
+    def edits(n):
+        do = vx.generate_primitives(depth + 2, n, 8, sphere_permille=500, add_permille=500,
+                                    r_min=1, r_max=128, log_uniform=True)
+        undo = do.copy()
+        undo["flags"] ^= 1 << 8
+        a, b = vx.prims_to_device(do, "cuda"), vx.prims_to_device(undo, "cuda")
+
+        def run():
+            dag.apply_primitives(a)
+            dag.apply_primitives(b)
+        return run
+
+    lanes = sweep("edit.leafparent_lanes", {f"{n} primitives": edits(n) for n in (1, 8, 32, 128)},
+                  lambda: dag.query(pts))
+
+    def strokes_and_scatter(world):
+        for r in strokes:
+            prim = np.zeros(1, vx.PRIM_DTYPE)
+            prim["c"][0] = (2 << depth) - 3
+            prim["r"][0, 0] = r
+            prim["flags"] = vx.make_flags(0, 1)
+            vox, _ = vx.rasterize(vx.prims_to_device(prim, "cuda"), depth + 2)
+            n = vox.shape[0]
+            scattered = torch.randint(0, 4 << depth, (n, 3), dtype=vox.dtype, device="cuda",
+                                      generator=g)
+            order = torch.randperm(n, device="cuda", generator=g)
+            for kind, v in (("stroke", vox[order].contiguous()), ("scattered", scattered)):
+                def run(v=v):
+                    if world.apply_voxels(v, 1) != 0 or world.apply_voxels(v, 0) != 0:
+                        raise RuntimeError("voxel list failed")
+                yield f"{type(world).__name__} {kind} {n}", run
+
+    voxels = sweep("edit.small_max_voxels",
+                   {**dict(strokes_and_scatter(dag)), **dict(strokes_and_scatter(svo))},
+                   lambda: torch.cat([dag.query(pts), svo.query(pts)]))
+    return {"edit.leafparent_lanes": lanes, "edit.small_max_voxels": voxels}, times
 
 
 def tune_serve(depth: int, scale: int, batch: int, reps: int, log, max_nodes: int,
@@ -251,8 +330,8 @@ def tune_serve(depth: int, scale: int, batch: int, reps: int, log, max_nodes: in
         log(f"  serve batch of {batch} blocks_per_sm={bps}: "
             + (f"{ms:.3f} ms" if ms is not None else "FAILED (not used)"))
     vx.reset_tuning()
-    valid = {int(k.split("=")[1]): t for k, t in times.items() if t is not None}
-    return {"serve.blocks_per_sm": min(valid, key=valid.get)}, times
+    valid = {int(k.split("=")[1]): t for k, t in times.items()}
+    return {"serve.blocks_per_sm": _pick(valid, vx.tuning()["serve.blocks_per_sm"])}, times
 
 
 def main(argv=None) -> dict:
@@ -270,11 +349,13 @@ def main(argv=None) -> dict:
         sort_best, sort_t = tune_sort(1 << 20, 1 << 19, 2, log)
         scan_best, scan_t = tune_scan(1 << 20, 2, log)
         edit_best, edit_t = tune_edit(6, 1, 256, 2, log, 1 << 18, 64 << 20)
+        small_best, small_t = tune_small(6, 1, (5, 12), 2, log, 1 << 18, 64 << 20)
         serve_best, serve_t = tune_serve(6, 1, 64, 2, log, 1 << 18, 64 << 20)
     else:
         sort_best, sort_t = tune_sort(1 << 26, 1 << 25, 5, log)
         scan_best, scan_t = tune_scan(1 << 28, 5, log)
         edit_best, edit_t = tune_edit(12, 64, 16384, 5, log, 1 << 27, 16 << 30)
+        small_best, small_t = tune_small(9, 8, (8, 12, 16, 20, 23), 15, log, 1 << 22, 2 << 30)
         serve_best, serve_t = tune_serve(11, 32, 400, 9, log, 1 << 27, 8 << 30)
     vx.reset_tuning()
     untuned = vx.tuning()  # knobs no sweep here times keep their defaults
@@ -282,8 +363,10 @@ def main(argv=None) -> dict:
         "device": dev,
         "quick": bool(args.quick),
         "seconds": round(time.time() - t0, 1),
-        "knobs": {**untuned, **sort_best, **scan_best, **edit_best, **serve_best},
-        "timings_ms": {"sort": sort_t, "scan": scan_t, "edit": edit_t, "serve": serve_t},
+        "knobs": {**untuned, **sort_best, **scan_best, **edit_best, **small_best,
+                  **serve_best},
+        "timings_ms": {"sort": sort_t, "scan": scan_t, "edit": edit_t, "small": small_t,
+                       "serve": serve_t},
     }
     out = args.out or str(tuning_file(dev))
     from pathlib import Path
