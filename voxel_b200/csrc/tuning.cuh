@@ -12,7 +12,7 @@ enum Id : uint32_t {
   kSortItemsU64,    // partition items per thread, u64 keys: 8 or 10
   kSortEarlyCounts, // publish tile digit counts before ranking: 0 or 1
   kSortRankBallots, // rank keys with per-bit ballots (1) or shared-memory atomic OR (0)
-  kEditBigItem,     // items with more primitives go to the block-per-item expansion
+  kEditBigItem,     // items with more primitives are expanded by a block or a cluster of blocks
   kEditBlocksPerSm, // grid of the edit pipelines' item kernels, in blocks per SM
   kEditLeafparentBlocks, // resident blocks the DAG leaf-parent kernel is built for
   kServeBlocksPerSm, // grid of the serving loop's edit graphs, in blocks per SM
@@ -21,7 +21,7 @@ enum Id : uint32_t {
   kEditSmallBlocksPerSm, // resident blocks per SM of that kernel
   kEditSmallMaxVoxels, // voxel lists / leaf commands of at most this length run that way
   kSortRadixBits,   // radix digit width in bits: 6, 7 or 8 (passes = key bits / width)
-  kScanTileKb,      // prefix-sum tile in KB: 32 (256 threads), 16 (128) or 8 (64)
+  kScanTileKb,      // prefix-sum tile in KB: 32, 16 (128 threads each) or 8 (64)
   kEditLeafparentPrefetch, // DAG leaf-parent kernel prefetches the next item's old node: 0 or 1
   kKnobCount
 };
