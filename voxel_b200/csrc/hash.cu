@@ -490,9 +490,11 @@ __device__ __forceinline__ bool cuckoo_claim(ulonglong2 *bucket, ulonglong2 e, u
 }
 
 // A key's first try: both buckets are read at once.  A key that is there is
-// replaced in the slot that was read; a new one takes a free slot of the
+// replaced (Direct: in the slot that was read; otherwise looked up again, for
+// the kernel that seldom meets one and lacks the registers); a new one takes a free slot of the
 // emptier bucket, so that fewer keys have to move later.  VX_HASH_OVERFLOW:
 // not settled, to be moved on from (key, *target, *rnd).
+template <bool Direct>
 __device__ __forceinline__ uint32_t cuckoo_try(ulonglong2 *slots, uint32_t nb, uint64_t key,
                                                uint32_t value, uint32_t &target, uint64_t &rnd) {
   if (key == kEmpty || key == kDeleted) return VX_HASH_INVALID_KEY;
@@ -512,11 +514,14 @@ __device__ __forceinline__ uint32_t cuckoo_try(ulonglong2 *slots, uint32_t nb, u
     if (v.x == kEmpty) free_slots |= 1u << j;
   }
   if (where != nullptr) {
-    const ulonglong2 seen = cas128(where, make_ulonglong2(key, word),
-                                   make_ulonglong2(key, (word & 0xffffffff00000000ull) | value));
+    bool done = false;
+    if (Direct) {
+      const ulonglong2 seen = cas128(where, make_ulonglong2(key, word),
+                                     make_ulonglong2(key, (word & 0xffffffff00000000ull) | value));
+      done = seen.x == key && seen.y == word;
+    }
     // (moved, or its value changed, meanwhile: looked up again)
-    if ((seen.x == key && seen.y == word) || cuckoo_replace(slots, nb, key, value))
-      return VX_HASH_REPLACED;
+    if (done || cuckoo_replace(slots, nb, key, value)) return VX_HASH_REPLACED;
   }
   rnd = mix64(key ^ 0x5851f42d4c957f2dull);
   const uint32_t room0 = __popc(free_slots & 3u), room1 = __popc(free_slots >> 2);
@@ -562,7 +567,7 @@ __global__ void __launch_bounds__(kBlock)
   ulonglong2 cur = make_ulonglong2(keys[i], values ? values[i] : static_cast<uint32_t>(i));
   uint32_t target = 0;
   uint64_t rnd = 0;
-  uint32_t status = cuckoo_try(slots, nb, cur.x, static_cast<uint32_t>(cur.y), target, rnd);
+  uint32_t status = cuckoo_try<true>(slots, nb, cur.x, static_cast<uint32_t>(cur.y), target, rnd);
   for (uint32_t moves = 0; status == VX_HASH_OVERFLOW; ++moves) {
     status = cuckoo_move(slots, nb, cur, target, rnd, moves);
     if (status == VX_HASH_OVERFLOW && moves >= max_evictions) {
@@ -609,7 +614,7 @@ __global__ void __launch_bounds__(kBlock, kCuckooBlocksPerSm)
         mine = static_cast<uint32_t>(take);
         cur = make_ulonglong2(keys[mine], values ? values[mine] : mine);
         const uint32_t status =
-            cuckoo_try(slots, nb, cur.x, static_cast<uint32_t>(cur.y), target, rnd);
+            cuckoo_try<false>(slots, nb, cur.x, static_cast<uint32_t>(cur.y), target, rnd);
         busy = status == VX_HASH_OVERFLOW;
         moves = 0;
         if (!busy && statuses) statuses[mine] = status;
