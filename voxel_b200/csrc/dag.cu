@@ -597,7 +597,8 @@ __device__ __forceinline__ void leafparent_warps(const Ctx &x, Blocks blk) {
 
 template <int MinBlocks, bool Prefetch>
 __global__ void __launch_bounds__(kBlock, MinBlocks) leafparent_kernel(Ctx x) {
-  if (x.t.hdr->item_count[x.t.depth - 1] <= kWideItems)
+  // (the same in every block; sorted leaf masks need no list walks)
+  if (x.sorted_keys == nullptr && x.t.hdr->item_count[x.t.depth - 1] <= kWideItems)
     leafparent_body<false, 8>(x, launch_blocks());
   else leafparent_warps<Prefetch, false>(x, launch_blocks());
 }
@@ -738,8 +739,8 @@ __global__ void __maxnreg__(255) small_edit_kernel(Ctx x, EditCtx e, PlainPrep p
     // blocks from the last one down, the short ones from block 0 up.
     expand_body<DagTree, false>(e, tree, l, blk);
     if (x.t.hdr->big_count[l] != 0)
-      expand_big_body<DagTree, false, kBlock, kSmallBigCache>(e, tree, l,
-                                                          Blocks{blk.count - 1u - blk.id, blk.count});
+      expand_big_body<DagTree, kBlock, kSmallBigCache>(e, tree, l,
+                                                   Blocks{blk.count - 1u - blk.id, blk.count});
     grid.sync();
   }
   // The bottom-up build without level barriers: the leaf-parent items and

@@ -339,7 +339,7 @@ struct Header {
   uint32_t pair_count[16];      // pairs of each level
   uint64_t node_count[16];      // items inserted per table (DAG)
   uint32_t pool_used[16];       // words used per level pool (DAG)
-  uint32_t big_count[16];       // items deferred to the block-per-item path
+  uint32_t big_count[16];       // items with long lists (EditCtx::big_item)
   uint32_t pool_mark[16];       // pool_used before this edit's inserts (DAG)
 };
 
@@ -353,8 +353,10 @@ struct Arena {
 };
 
 // Items with more primitives than EditCtx::big_item (the tuning knob
-// "edit.big_item", 32 by default) are expanded by a whole block.  They are
-// listed when they are emitted (the level above's expansion, or the init of
+// "edit.big_item", 32 by default) are expanded apart: in batches by
+// expand_long_kernel (a cluster of eight blocks above 4,096 primitives, a block
+// below), in small edits by a block (expand_big_body).  They are listed when
+// they are emitted (the level above's expansion, or the init of
 // the root), so that a level's short and long lists can be expanded side by
 // side; the big buffer's two halves alternate by level, so level l + 1's
 // list fills while level l's is read.
@@ -374,7 +376,7 @@ struct EditCtx {
   const uint32_t *d_prim_count; // device count (NULL: use host_prim_count)
   uint32_t host_prim_count;
   uint32_t depth;
-  uint32_t big_item; // longer primitive lists go to expand_big_kernel
+  uint32_t big_item; // items with longer primitive lists are listed (big_list)
   // Not NULL: the primitives are leaf masks of distinct leaves in ascending
   // leaf key (Morton) order, with these keys, so an item's list is a range of
   // them (expand_sorted_body).
@@ -382,7 +384,7 @@ struct EditCtx {
 };
 
 // List item `idx` of level l (its index within the level) for the
-// block-per-item expansion when its primitive list is long and level l is
+// long lists' expansion when its primitive list is long and level l is
 // expanded at all (levels below depth - 1).
 __device__ __forceinline__ void note_big(const EditCtx &x, uint32_t l, uint32_t idx,
                                          uint32_t pcount) {
@@ -616,8 +618,7 @@ __device__ __forceinline__ void expand_body(EditCtx x, Policy pol, uint32_t l, B
     const bool have = wi < W;
     Item it{};
     if (have) it = x.a.items[base + wi];
-    // Long lists were listed for expand_big (one block per item) when the
-    // item was emitted.
+    // Items with long lists were listed when they were emitted (big_list).
     const bool big = have && it.pcount > x.big_item;
     if (big) it.pcount = 0;
     const Cell cell = unpack_cell(it.cell);
@@ -835,7 +836,7 @@ __global__ void __launch_bounds__(kBlock, 4) expand_warp_kernel(EditCtx x, Polic
     const bool have = w0 + lane < W;
     Item it{};
     if (have) it = x.a.items[base + wi];
-    // Long lists were listed for expand_big when the item was emitted.
+    // Items with long lists were listed when they were emitted (big_list).
     const bool big = have && it.pcount > x.big_item;
     const bool single = have && it.pcount == 1u;
     uint32_t v = 0, npairs = 0, pidx = 0;
@@ -1049,8 +1050,8 @@ __global__ void __launch_bounds__(kBlock, 4) expand_warp_kernel(EditCtx x, Polic
 //
 // Walking the lists costs time in proportion to the list at every level whose
 // cells hold most of it, on one block per cell: the 144,000 leaves of a
-// sphere of radius 128 in a 4096^3 world took expand_big_kernel 5.8 ms (and
-// expand_kernel 0.18 ms) of an edit's 7.0 ms on B200, the searches 0.10 ms (by
+// sphere of radius 128 in a 4096^3 world took a block per cell 5.8 ms (and
+// the short lists 0.18 ms) of an edit's 7.0 ms on B200, the searches 0.10 ms (by
 // halves 0.13): a chain of log8(list) round trips to L2 per level.
 template <class Policy>
 __device__ __forceinline__ void expand_sorted_body(EditCtx x, Policy pol, uint32_t l, Blocks blk) {
@@ -1151,7 +1152,7 @@ inline uint32_t level_grid(uint32_t grid, uint32_t l, uint32_t per_block) {
 // block-wide compaction of those into each child's list.  Lists of up to
 // Cache primitives are classified once: walk 1 keeps each primitive's
 // per-child MIXED bits in shared memory for walks 2 and 3.
-template <class Policy, bool Terrain, uint32_t Threads, uint32_t Cache>
+template <class Policy, uint32_t Threads, uint32_t Cache>
 __device__ __forceinline__ void expand_big_body(EditCtx x, Policy pol, uint32_t l, Blocks blk) {
   Header *h = x.hdr;
   // the level's counts and this block's first listed item load beside the
@@ -1203,7 +1204,7 @@ __device__ __forceinline__ void expand_big_body(EditCtx x, Policy pol, uint32_t 
         const int64_t ox = int64_t(2 * cell.x + (c & 1u)) * csize;
         const int64_t oy = int64_t(2 * cell.y + ((c >> 1) & 1u)) * csize;
         const int64_t oz = int64_t(2 * cell.z + ((c >> 2) & 1u)) * csize;
-        const uint32_t cls = pol.template classify<Terrain>(pr, world_exp, ox, oy, oz, csize);
+        const uint32_t cls = pol.template classify<false>(pr, world_exp, ox, oy, oz, csize);
         if (cls == VX_CELL_FULL) last[c] = max(last[c], static_cast<int32_t>(p));
         else if (cls == VX_CELL_MIXED) mixed |= 1u << c;
       }
@@ -1235,7 +1236,7 @@ __device__ __forceinline__ void expand_big_body(EditCtx x, Policy pol, uint32_t 
         const int64_t ox = int64_t(2 * cell.x + (c & 1u)) * csize;
         const int64_t oy = int64_t(2 * cell.y + ((c >> 1) & 1u)) * csize;
         const int64_t oz = int64_t(2 * cell.z + ((c >> 2) & 1u)) * csize;
-        if (pol.template classify<Terrain>(pr, world_exp, ox, oy, oz, csize) == VX_CELL_MIXED) ++cnt[c];
+        if (pol.template classify<false>(pr, world_exp, ox, oy, oz, csize) == VX_CELL_MIXED) ++cnt[c];
       }
     }
 #pragma unroll
@@ -1310,7 +1311,7 @@ __device__ __forceinline__ void expand_big_body(EditCtx x, Policy pol, uint32_t 
           const int64_t ox = int64_t(2 * cell.x + (c & 1u)) * csize;
           const int64_t oy = int64_t(2 * cell.y + ((c >> 1) & 1u)) * csize;
           const int64_t oz = int64_t(2 * cell.z + ((c >> 2) & 1u)) * csize;
-          if (pol.template classify<Terrain>(pr, world_exp, ox, oy, oz, csize) == VX_CELL_MIXED)
+          if (pol.template classify<false>(pr, world_exp, ox, oy, oz, csize) == VX_CELL_MIXED)
             take |= 1u << c;
         }
       }

@@ -377,7 +377,8 @@ __global__ void __launch_bounds__(kBlock, Mats ? 3 : 4) leafparent_kernel(EditCt
   const uint32_t W = h->item_count[l]; // loaded beside the status
   const uint32_t base = h->item_off[l];
   if (edit_failed(h)) return;
-  if (W <= kWideItems) { // the same in every block
+  // (the same in every block; sorted leaf masks need no list walks)
+  if (x.sorted_keys == nullptr && W <= kWideItems) {
     leafparent_body<false>(x, t, launch_blocks());
     return;
   }
@@ -890,8 +891,8 @@ __global__ void __maxnreg__(255) small_edit_kernel(EditCtx e, Tables t, PlainPre
     // blocks from the last one down, the short ones from block 0 up.
     expand_body<SvoTree, false>(e, pol, l, blk);
     if (t.hdr->big_count[l] != 0)
-      expand_big_body<SvoTree, false, kBlock, kSmallBigCache>(e, pol, l,
-                                                          Blocks{blk.count - 1u - blk.id, blk.count});
+      expand_big_body<SvoTree, kBlock, kSmallBigCache>(e, pol, l,
+                                                   Blocks{blk.count - 1u - blk.id, blk.count});
     grid.sync();
   }
   // Every block reaches the capacity verdict from the
