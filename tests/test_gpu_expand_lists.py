@@ -1,6 +1,8 @@
 """Batched expansion around its list lengths: items with one primitive, with a
 few (up to 32 and beyond), long lists on one block and on a cluster of blocks
-(4,096), lists past a block's kept bits, mixed shapes, against the oracle."""
+(4,096), lists past the bits that a cluster keeps (262,144), mixed shapes, on
+both sides of the level size from which a lane takes an item, against the
+oracle."""
 import numpy as np
 import pytest
 
@@ -44,6 +46,59 @@ def test_list_lengths_match_oracle(cuda, kind, n):
         assert svo.status() == 0
         assert (oracle.SvoCanon(*svo.canonical())
                 == oracle.Grid(depth, materials=mats).apply_prims(p).svo())
+
+
+@pytest.mark.parametrize("kind", ["spheres", "mixed"])
+def test_a_list_past_the_kept_bits_matches_oracle(cuda, kind):
+    n = 270_001  # 8 blocks keep 32,768 primitives' bits each
+    rng = np.random.default_rng(n)
+    depth = 5
+    p = prims(kind, n, 4 << depth, rng)
+    p["r"][rng.random(n) < 0.9] = 0  # mostly single voxels: the oracle applies all of them
+    d = vx.prims_to_device(p, cuda)
+    dag = vx.HashDag(depth, 1 << 18, 512 << 20)
+    dag.apply_primitives(d)
+    assert dag.status() == 0
+    svo = vx.Svo(depth, 1 << 18, 1 << 18, materials=True, arena_bytes=512 << 20)
+    svo.apply_primitives(d)
+    assert svo.status() == 0
+    assert oracle.DagCanon(*dag.canonical()) == oracle.Grid(depth).apply_prims(p).dag()
+    assert (oracle.SvoCanon(*svo.canonical())
+            == oracle.Grid(depth, materials=True).apply_prims(p).svo())
+
+
+@pytest.mark.parametrize("n", [300, 12000])
+@pytest.mark.parametrize("boxes", [False, True])
+def test_levels_of_few_and_many_items_match_oracle(cuda, n, boxes):
+    """A crowd (few items, several primitives each) and primitives all over
+    the world (levels of more than 37,888 items) on a 512^3 world."""
+    depth = 7
+    world = 4 << depth
+    rng = np.random.default_rng(n + boxes)
+    p = np.zeros(n, oracle.PRIM_DTYPE)
+    if n == 300:
+        p["c"] = world // 2 + rng.integers(-32, 32, (n, 3))
+        r = rng.integers(4, 28, (n, 3))
+    else:
+        p["c"] = rng.integers(0, world, (n, 3))
+        r = rng.integers(2, 9, (n, 3))
+    p["r"] = r if boxes else r * [1, 0, 0]
+    op = rng.integers(0, 2, n)
+    p["flags"] = int(boxes) | (op << 8) | ((rng.integers(1, 4, n) * op) << 16)
+    d = vx.prims_to_device(p, cuda)
+    dag = vx.HashDag(depth, 1 << 21, 1 << 30)
+    dag.build_terrain(3, 2, True)
+    dag.apply_primitives(d)
+    assert dag.status() == 0
+    t = oracle.terrain(seed=3, scale=2, caves=True)
+    assert (oracle.DagCanon(*dag.canonical())
+            == oracle.Grid(depth).terrain(t).apply_prims(p).dag())
+    svo = vx.Svo(depth, 1 << 20, 1 << 22, materials=True, arena_bytes=1 << 30)
+    svo.build_terrain(3, 2, True)
+    svo.apply_primitives(d)
+    assert svo.status() == 0
+    assert (oracle.SvoCanon(*svo.canonical())
+            == oracle.Grid(depth, materials=True).terrain(t).apply_prims(p).svo())
 
 
 def test_failed_edit_leaves_every_cluster(cuda):
