@@ -32,6 +32,13 @@ struct GroupRecords32 {
 constexpr uint32_t kGroup = 32, kGroupCount = 40;
 constexpr uint64_t kReady = 1ull << 63;
 
+__device__ __forceinline__ void publish_group(const GroupRecords32 &r, uint32_t tile,
+                                              uint32_t aggregate) {
+  atomicAdd(reinterpret_cast<unsigned long long *>(r.group_sum + tile / kGroup),
+            (1ull << kGroupCount) + aggregate);
+  st_relaxed_u64(r.tile + tile, kReady | aggregate);
+}
+
 // Look-back for u32 sums, called by one full warp after lane 0 published the
 // tile (publish_group): lane l reads the record of its group's tile l and the
 // words of the l-th group back, until the tiles before it in its group and the
@@ -40,13 +47,6 @@ constexpr uint64_t kReady = 1ull << 63;
 // the inclusive prefix of the group before its own, so every tile ends.
 // Returns the sum of all earlier tiles (in every lane); on timeout sets
 // *status and returns a partial sum.
-__device__ __forceinline__ void publish_group(const GroupRecords32 &r, uint32_t tile,
-                                              uint32_t aggregate) {
-  atomicAdd(reinterpret_cast<unsigned long long *>(r.group_sum + tile / kGroup),
-            (1ull << kGroupCount) + aggregate);
-  st_relaxed_u64(r.tile + tile, kReady | aggregate);
-}
-
 __device__ __forceinline__ uint32_t group_lookback(const GroupRecords32 &r, uint32_t tile,
                                                    uint32_t aggregate, uint32_t *status) {
   const uint32_t lane = lane_id();
@@ -110,10 +110,11 @@ template <> struct RecordsFor<uint32_t> { using type = GroupRecords32; };
 template <> struct RecordsFor<uint64_t> { using type = SplitRecords64; };
 
 // Warp-parallel look-back for u64 sums, called by one full warp after lane 0
-// published the tile's aggregate (publish_tile).  Reads the records of the previous 32 * R tiles at once
-// (lane l, row j reads distance l + 32 j: R coalesced loads in flight per
-// lane), accumulates back to the nearest inclusive record, publishes the
-// inclusive prefix and returns the exclusive prefix (valid in every lane).
+// published the tile's aggregate (SplitRecords64::publish).  Reads the records
+// of the previous 32 * R tiles at once (lane l, row j reads distance l + 32 j:
+// R coalesced loads in flight per lane), accumulates back to the nearest
+// inclusive record, publishes the inclusive prefix and returns the exclusive
+// prefix (valid in every lane).
 // A window wider than one warp matters because with hundreds of tiles
 // resident the nearest inclusive record can be far back, and each window
 // costs one round trip to L2.  On timeout sets *status and returns a partial
