@@ -10,7 +10,7 @@ import oracle
 import voxel_b200 as vx
 
 pytestmark = pytest.mark.gpu
-FEWEST = 1 << 17
+FEWEST = 3 << 17
 
 
 def grouped_rays(rng, n, world):
@@ -36,7 +36,7 @@ def grouped_rays(rng, n, world):
     return r
 
 
-@pytest.mark.parametrize("n", [31, FEWEST, FEWEST + 1, FEWEST + 32, 300_001])
+@pytest.mark.parametrize("n", [31, FEWEST, FEWEST + 1, FEWEST + 32, 500_001])
 def test_grouped_rays_match_oracle(cuda, n):
     depth = 6
     world = 4 << depth

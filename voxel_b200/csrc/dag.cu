@@ -772,9 +772,9 @@ __global__ void query_kernel(vx_dag_view v, const vx_voxel *pts, uint32_t n,
 // Rays differ in length by orders of magnitude (a miss of the world, a ray
 // along a cave).  Two kernels share a list of rays, 32 at a time:
 //
-// raycast_kernel, a thread per ray, takes those whose 32 rays are alike
-// (primary rays of neighbouring pixels): they walk the same cells, so the
-// warp stays together, and its blocks are dealt out as others end.
+// raycast_kernel, a thread per ray, takes short lists and those groups whose 32
+// rays are alike (primary rays of neighbouring pixels): they walk the same
+// cells, so the warp stays together, and its blocks are dealt out as others end.
 //
 // raycast_refill_kernel takes the others.  A thread per ray would leave a warp
 // waiting for its longest (5.75 of 32 lanes were active per instruction), so
@@ -788,11 +788,13 @@ __global__ void query_kernel(vx_dag_view v, const vx_voxel *pts, uint32_t n,
 //   images of 1024^2 rays from three eyes  393 530 293 / 461 713 305 / 416 548 302
 //   images of 2048^2 rays                861 1442 520 / 1221 2079 698 / 900 1490 575
 //   65,536 rays                                               209 / 225 / -
-// Up to kRayFewest rays, which all run at once, are alike for this purpose:
-// the longest decides.  (Refilling at 16 and 24 idle lanes, 2 and 8 steps
-// between refills, 4 and 6 blocks per SM: 600-800 us for the first.)
+//   350,000 such rays, five seeds: 344-494 a thread per ray, 411-491 both kernels
+//   440,000: 391-505, 392-480; 700,000: 560-639, 472-524
+// Up to kRayFewest rays the longest decide: a thread per ray.  (Refilling at 4,
+// 16 and 24 idle lanes, 2 and 8 steps between refills, 4 and 6 blocks per SM:
+// 590-800 us for the first.)
 constexpr uint32_t kRayRefill = 8, kRaySteps = 4, kRayBlocksPerSm = 5;
-constexpr uint32_t kRayFewest = 1u << 17;
+constexpr uint32_t kRayFewest = 3u << 17;
 
 // Whether the 32 rays from `first` on are alike: directions within 11.5 degrees
 // (cos^2 0.96) of the first one's and origins within a sixteenth of the world
