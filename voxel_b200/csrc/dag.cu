@@ -1158,7 +1158,7 @@ vx_status run_pipeline(vx_dag *d, const vx_primitive *prims,
         expand_sorted_kernel<DagTree><<<lgrid, kBlock, 0, s>>>(e, tree, l);
       else
         expand_warp_kernel<DagTree>
-            <<<lgrid, kBlock, 0, s>>>(e, tree, l);
+            <<<expand_grid(grid, l), kBlock, 0, s>>>(e, tree, l);
     }
     VX_TRY_CUDA(cudaGetLastError());
     if (sorted_keys != nullptr || terrain) continue; // no long lists

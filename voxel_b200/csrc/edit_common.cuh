@@ -1145,6 +1145,13 @@ inline uint32_t level_grid(uint32_t grid, uint32_t l, uint32_t per_block) {
   return need < grid ? need : grid;
 }
 
+// Blocks of expand_warp_kernel for level l: 256 items a block, or 32 while the
+// level has so few that it takes the eight-lane body.
+inline uint32_t expand_grid(uint32_t grid, uint32_t l) {
+  return std::max(level_grid(grid, l, kBlock),
+                  std::min(level_grid(grid, l, kBlock / 8), ceil_div(kWideItems, kBlock / 8)));
+}
+
 // Expansion of the long-list items of level l inside the small cooperative
 // kernels: one block of Threads threads per item.  Three walks over the list:
 // the last fully-covering primitive per child (block max), the partial

@@ -1047,7 +1047,7 @@ vx_status run_pipeline(vx_svo *v, const vx_primitive *prims, const uint32_t *d_c
       else if (sorted_keys) expand_sorted_kernel<SvoTree><<<lgrid, kBlock, 0, s>>>(e, pol, l);
       else
         expand_warp_kernel<SvoTree>
-            <<<lgrid, kBlock, 0, s>>>(e, pol, l);
+            <<<expand_grid(grid, l), kBlock, 0, s>>>(e, pol, l);
     }
     VX_TRY_CUDA(cudaGetLastError());
     if (sorted_keys != nullptr || terrain) continue; // no long lists
