@@ -778,9 +778,9 @@ __global__ void __launch_bounds__(kBlock)
 // lists four (expansion) or a leaf at a time (leaf parents) while most of the
 // chip has nothing to do.  B200, us, one lane / eight lanes up to here (eight
 // always): 2,000 spheres of radius 16-64 with their centres in a 256^3 part
-// of a 2048^3 Hash DAG 620 / 377 (453), of an SVO 578 / 390 (594); 1,000
+// of a 2048^3 Hash DAG 620 / 369 (453), of an SVO 578 / 371 (594); 1,000
 // primitives in a 256^3 world 393 / 187 (287); 8,000 spheres all over 2048^3
-// 592 / 470 (893).
+// 592 / 463 (893).
 constexpr uint32_t kWideItems = 37888; // 148 multiprocessors x 256 groups of eight
 
 // expand_body for the batches' own launches: a warp takes 32 items at a time
